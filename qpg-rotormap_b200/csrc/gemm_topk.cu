@@ -17,8 +17,9 @@
 //   warps 2..5  epilogue: one thread per read row (TMEM lane); tcgen05.ld of
 //               32 columns at a time (the next chunk in flight while one is
 //               scored), score transform (fp16 rounding / column scale),
-//               chunk max vs the row's threshold, and insertion into a
-//               register reservoir of the top KT (score desc, column asc).
+//               group maxima vs the row's threshold, candidates buffered in
+//               shared memory and inserted in bulk into a register reservoir
+//               of the top KT (score desc, column asc).
 // Work unit = (read tile of 128 rows, column split); each unit streams its
 // split's column tiles and leaves a sorted partial list per row; a second
 // kernel merges the splits.  Every mbarrier wait is bounded; a wait that
@@ -57,7 +58,10 @@ constexpr int MAX_SPLITS = 128;
 // per launch (epi_halves_for).  KT = 64 always uses H = 1 (its reservoir
 // needs the registers).
 __host__ __device__ constexpr int epi_threads(int H) { return 64 + 128 * H; }
-constexpr int SCRATCH_F = 17;  // floats per epilogue thread (16-value slow-path passes)
+// Candidate buffer of the epilogue: 32 KiB per CTA (what the operand stages
+// leave of shared memory), entry e of epilogue thread t at [e][t].
+constexpr int CAND_BYTES = 32 * 1024;
+__host__ __device__ constexpr int cand_cap(int H) { return CAND_BYTES / 8 / (128 * H); }  // entries per thread
 // 256-column tiles per work unit at or below which the 8-warp epilogue pays
 constexpr int SHORT_UNIT_TILES = 8192;
 
@@ -69,6 +73,7 @@ struct GemmArgs {
   int splits;
   int num_kb;
   int score_mode;
+  int k;     // results wanted per row (<= KT)
   int mpad;  // num_m_tiles * BM (partial-list row stride)
   const float *scaleB;
   float *part_vals;
@@ -86,9 +91,7 @@ __device__ __forceinline__ float round_f16(float x) { return __half2float(__floa
 
 // The best KT (value, column) pairs of one row, kept sorted in registers:
 // larger value first, equal values -> smaller column first.  `thr` is the
-// worst kept value.  Insertion is branch-free: the new entry's rank is a sum
-// of independent compares and every slot picks (old, shifted, new) with two
-// selects, so there is no dependent chain through the list.
+// k-th of them: a later column has to beat it to enter the row's top k.
 template <int KT>
 struct Reservoir {
   float v[KT];
@@ -103,25 +106,80 @@ struct Reservoir {
     }
     thr = -INFINITY;
   }
-  // Called only with x > thr and a column larger than every kept column (the
-  // scan runs in increasing column order), so the rank is #{v[i] >= x}.
+  // Columns arrive in increasing order, so an equal value goes behind the
+  // kept one.  x <= v[KT-1] (-inf, a candidate that has since been beaten)
+  // changes nothing.  Every slot picks (old, shifted, new) from two compares:
+  // no chain through the list.
   __device__ __forceinline__ void insert(float x, int col) {
-    int p = 0;
-#pragma unroll
-    for (int i = 0; i < KT; ++i) p += (v[i] >= x) ? 1 : 0;
+    bool above = x > v[KT - 1];
 #pragma unroll
     for (int i = KT - 1; i > 0; --i) {
-      const bool shift = i > p, here = i == p;
-      v[i] = shift ? v[i - 1] : (here ? x : v[i]);
-      c[i] = shift ? c[i - 1] : (here ? col : c[i]);
+      const bool next = x > v[i - 1];
+      v[i] = above ? (next ? v[i - 1] : x) : v[i];
+      c[i] = above ? (next ? c[i - 1] : col) : c[i];
+      above = next;
     }
-    if (p == 0) {
+    if (above) {
       v[0] = x;
       c[0] = col;
     }
-    thr = v[KT - 1];
   }
-  __device__ __forceinline__ void sort_desc() {}
+  // v[k-1] by selects (a run-time index would move the list to memory)
+  __device__ __forceinline__ void update_thr(int k) {
+    thr = v[0];
+#pragma unroll
+    for (int i = 1; i < KT; ++i) thr = i < k ? v[i] : thr;
+  }
+};
+
+// Candidates of one row waiting to enter its reservoir.  An insertion costs
+// a warp ~5 KT instructions whether one lane or all 32 have a candidate, and
+// the lanes' rows find theirs in different columns.  So a column that beats
+// its row's threshold is appended to the lane's buffer in shared memory (a
+// predicated store), and once a lane's buffer could overflow on the next 8
+// columns the warp empties all of them together, entry by entry: one
+// insertion then serves most of the lanes.  The threshold stands still
+// meanwhile, which only lets a few more candidates in; each is compared again
+// when it is inserted.  This bounds every search whose units are short: about
+// KT ln(columns / KT) insertions a row, against 32 cycles of MMA a column.
+// Inserting column by column as they came, rdim 2048, fused kernel alone:
+// 1,000 reads x 300,007 columns 2,346 us -> 614 us, 8,192 x 50,000 3,159 ->
+// 750, 4,096 x 500,000 at k = 64 50.1 ms -> 5.0 ms, 65,536 x 1,048,576
+// 122.0 -> 100.3 ms.
+template <int H>
+struct Candidates {
+  static constexpr uint32_t STRIDE = 128 * H * 8;  // bytes between a thread's entries
+  uint32_t base, end, limit;
+
+  __device__ __forceinline__ void init(uint32_t smem_base, int t) {
+    base = end = smem_base + 8u * (uint32_t)t;
+    limit = base + STRIDE * (uint32_t)(cand_cap(H) - 8);
+  }
+  __device__ __forceinline__ void append(float x, float thr, int col) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.gt.f32 p, %1, %2;\n\t"
+        "@p st.shared.v2.b32 [%0], {%3, %4};\n\t"
+        "@p add.u32 %0, %0, %5;\n\t}"
+        : "+r"(end)
+        : "f"(x), "f"(thr), "r"(__float_as_uint(x)), "r"(col), "n"(STRIDE)
+        : "memory");
+  }
+  // Called by the whole warp.
+  template <int KT>
+  __device__ __forceinline__ void flush(Reservoir<KT> &R, int k) {
+    const unsigned FULL = 0xFFFFFFFFu;
+    const uint32_t most = __reduce_max_sync(FULL, end - base);
+#pragma unroll 1
+    for (uint32_t o = 0; o < most; o += STRIDE) {
+      uint32_t xb = 0xFF800000u, col = 0;  // -inf: no candidate
+      if (base + o < end)
+        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(xb), "=r"(col) : "r"(base + o) : "memory");
+      R.insert(__uint_as_float(xb), (int)col);
+    }
+    end = base;
+    R.update_thr(k);
+  }
 };
 
 // Column scales of one 32-column chunk: broadcast loads (every lane of the
@@ -155,37 +213,34 @@ __device__ __forceinline__ void apply_scales(float (&v)[32], const float4 (&s)[8
   }
 }
 
-// Score one 32-column chunk of this thread's row (columns c0 .. c0+31): the
-// chunk max (a depth-5 tree over 8 partial maxima) against the row's threshold decides whether the
-// chunk goes through the insert path, staged 16 values at a time in `scratch`.
-template <int KT>
-__device__ __forceinline__ void score_chunk(Reservoir<KT> &R, float (&v)[32], long long c0, long long N, bool tail,
-                                            bool f16, float *scratch) {
+// Score one 32-column chunk of this thread's row (columns c0 .. c0+31).  The
+// maxima of its four groups of 8 columns against the row's threshold decide,
+// for the warp as a whole, which groups have candidates.
+template <int KT, int H>
+__device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, float (&v)[32], long long c0,
+                                            long long N, bool tail, bool f16, int k) {
+  const unsigned FULL = 0xFFFFFFFFu;
   if (tail) {
 #pragma unroll
     for (int j = 0; j < 32; ++j)
       if (c0 + j >= N) v[j] = -INFINITY;
   }
-  float m[8];
+  float m[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) m[j] = fmaxf(fmaxf(v[j], v[j + 8]), fmaxf(v[j + 16], v[j + 24]));
-#pragma unroll
-  for (int w = 4; w >= 1; w >>= 1)
-#pragma unroll
-    for (int j = 0; j < w; ++j) m[j] = fmaxf(m[j], m[j + w]);
-  float mx = m[0];
+  for (int q = 0; q < 4; ++q) {
+    const float *w = v + 8 * q;
+    m[q] = fmaxf(fmaxf(fmaxf(w[0], w[1]), fmaxf(w[2], w[3])), fmaxf(fmaxf(w[4], w[5]), fmaxf(w[6], w[7])));
+  }
+  float mx = fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
   if (f16) mx = round_f16(mx);
-  if (mx > R.thr) {
+  if (!__any_sync(FULL, mx > R.thr)) return;
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
+  for (int q = 0; q < 4; ++q) {
+    if (f16) m[q] = round_f16(m[q]);
+    if (__any_sync(FULL, m[q] > R.thr)) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) scratch[j] = v[16 * p + j];
-#pragma unroll 1
-      for (int j = 0; j < 16; ++j) {
-        float x = scratch[j];
-        if (f16) x = round_f16(x);
-        if (x > R.thr) R.insert(x, (int)(c0 + 16 * p + j));
-      }
+      for (int j = 8 * q; j < 8 * q + 8; ++j) Q.append(f16 ? round_f16(v[j]) : v[j], R.thr, (int)(c0 + j));
+      if (__any_sync(FULL, Q.end > Q.limit)) Q.flush(R, k);
     }
   }
 }
@@ -195,9 +250,9 @@ __device__ __forceinline__ void score_chunk(Reservoir<KT> &R, float (&v)[32], lo
 // into the row's reservoir.  Software-pipelined: the TMEM load and the column
 // scales of chunk i + 1 are in flight while chunk i is scored.  Every load is
 // waited for before returning, so the caller may release the accumulator.
-template <int KT, int CH>
-__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, uint32_t taddr, long long c_first, long long N,
-                                           const float *scaleB, bool scaled, bool f16, float *scratch) {
+template <int KT, int H, int CH>
+__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+                                           const float *scaleB, bool scaled, bool f16, int k) {
   static_assert(CH % 2 == 0, "chunks are drained in pairs");
   const bool tail = c_first + 32LL * CH > N;
   float va[32], vb[32];
@@ -213,7 +268,7 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, uint32_t taddr, lon
     if (scaled) apply_scales(va, s);
     tmem_ld32(taddr + (uint32_t)(i + 1) * 32u, vb);
     if (scaled) load_scales(s, scaleB, c0 + 32, N, tail);
-    score_chunk(R, va, c0, N, tail, f16, scratch);
+    score_chunk(R, Q, va, c0, N, tail, f16, k);
     __syncwarp();
     tmem_wait_ld_tied(vb);
     if (scaled) apply_scales(vb, s);
@@ -221,15 +276,16 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, uint32_t taddr, lon
       tmem_ld32(taddr + (uint32_t)(i + 2) * 32u, va);
       if (scaled) load_scales(s, scaleB, c0 + 64, N, tail);
     }
-    score_chunk(R, vb, c0 + 32, N, tail, f16, scratch);
+    score_chunk(R, Q, vb, c0 + 32, N, tail, f16, k);
   }
 }
 
-// The same, one chunk at a time: for the 8-warp form with a 32-entry
-// reservoir, whose 168-register budget has no room for a second chunk.
-template <int KT, int CH>
-__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, uint32_t taddr, long long c_first, long long N,
-                                                  const float *scaleB, bool scaled, bool f16, float *scratch) {
+// The same, one chunk at a time: for the 8-warp form, whose 168-register
+// budget has no room for a second chunk (two warps per scheduler cover the
+// TMEM latency), and for the 64-entry reservoir.
+template <int KT, int H, int CH>
+__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+                                                  const float *scaleB, bool scaled, bool f16, int k) {
   const bool tail = c_first + 32LL * CH > N;
 #pragma unroll 1
   for (int i = 0; i < CH; ++i) {
@@ -241,18 +297,18 @@ __device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, uint32_t tad
     tmem_ld32(taddr + (uint32_t)i * 32u, v);
     tmem_wait_ld_tied(v);
     if (scaled) apply_scales(v, s);
-    score_chunk(R, v, c0, N, tail, f16, scratch);
+    score_chunk(R, Q, v, c0, N, tail, f16, k);
   }
 }
 
 template <int KT, int H>
-__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, uint32_t taddr, long long c_first, long long N,
-                                      const float *scaleB, bool scaled, bool f16, float *scratch) {
+__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+                                      const float *scaleB, bool scaled, bool f16, int k) {
   constexpr int CH = BN / 32 / H;
-  if constexpr (H == 1 || KT < 32)
-    drain_tile<KT, CH>(R, taddr, c_first, N, scaleB, scaled, f16, scratch);
+  if constexpr (H == 1 && KT < 64)
+    drain_tile<KT, H, CH>(R, Q, taddr, c_first, N, scaleB, scaled, f16, k);
   else
-    drain_tile_serial<KT, CH>(R, taddr, c_first, N, scaleB, scaled, f16, scratch);
+    drain_tile_serial<KT, H, CH>(R, Q, taddr, c_first, N, scaleB, scaled, f16, k);
 }
 
 template <int KT, int H>
@@ -271,7 +327,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   uint64_t *drain = acc_empty + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  float *scratch_all = reinterpret_cast<float *>(tmem_slot + 4);  // epilogue threads x SCRATCH_F floats
+  const uint32_t cand = smem_u32(tmem_slot + 4);  // candidate buffers (CAND_BYTES)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
@@ -411,13 +467,14 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     const int quarter = warp & 3;    // TMEM lanes [32*quarter, 32*quarter+32)
     const int half = (warp - 2) >> 2;  // tile chunks [CH half, CH half + CH)
     const int row_in_tile = quarter * 32 + lane;
-    float *scratch = scratch_all + (threadIdx.x - 64) * SCRATCH_F;
     const bool f16 = g.score_mode == R2M_SCORE_F16;
     const bool scaled = g.score_mode == R2M_SCORE_SCALED;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     Reservoir<KT> R;
+    Candidates<H> Q;
+    Q.init(cand, threadIdx.x - 64);
     for (int u = blockIdx.x; ok && u < num_units; u += gridDim.x) {
       const int mt = u % g.num_m_tiles, sp = u / g.num_m_tiles;
       const int t0 = split_lo(sp, g.n_tiles, g.splits), t1 = split_lo(sp + 1, g.n_tiles, g.splits);
@@ -432,7 +489,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, scratch);
+        drain_acc<KT, H>(R, Q, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -440,7 +497,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         if (acc == 0) acc_phase ^= 1u;
       }
       if (!ok) break;
-      R.sort_desc();
+      Q.flush(R, g.k);
       const int row = mt * BM + row_in_tile;
       if (row < g.nb) {
         const size_t list = (size_t)sp * H + half;
@@ -546,7 +603,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   uint64_t *drain = acc_empty + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  float *scratch_all = reinterpret_cast<float *>(tmem_slot + 4);  // epilogue threads x SCRATCH_F floats
+  const uint32_t cand = smem_u32(tmem_slot + 4);  // candidate buffers (CAND_BYTES)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
@@ -708,13 +765,14 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     const int quarter = warp & 3;          // TMEM lanes this warp may read
     const int half = (warp - 2) >> 2;      // tile chunks [CH half, CH half + CH)
     const int row_in_tile = quarter * 32 + lane;
-    float *scratch = scratch_all + (threadIdx.x - 64) * SCRATCH_F;
     const bool f16 = g.score_mode == R2M_SCORE_F16;
     const bool scaled = g.score_mode == R2M_SCORE_SCALED;
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
     Reservoir<KT> R;
+    Candidates<H> Q;
+    Q.init(cand, threadIdx.x - 64);
     for (int u = pair; ok && u < num_units; u += npairs) {
       const int mt = u % g.num_m_tiles, sp = u / g.num_m_tiles;
       const int t0 = split_lo(sp, g.n_tiles, g.splits), t1 = split_lo(sp + 1, g.n_tiles, g.splits);
@@ -729,7 +787,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, scratch);
+        drain_acc<KT, H>(R, Q, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), 0));
@@ -737,6 +795,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         if (acc == 0) acc_phase ^= 1u;
       }
       if (!ok) break;
+      Q.flush(R, g.k);
       const int row = mt * 256 + (int)rank * 128 + row_in_tile;
       if (row < g.nb) {
         const size_t list = (size_t)sp * H + half;
@@ -886,7 +945,7 @@ static int pick_kt(int k) {
 
 static size_t gemm_smem_bytes(int H) {
   return 1024 + (size_t)STAGES * (A_STAGE + B_STAGE) + (2 * STAGES + 5) * 8 + 16 +
-         (size_t)(epi_threads(H) - 64) * SCRATCH_F * sizeof(float);
+         CAND_BYTES;
 }
 
 // Column splits for a given number of read tiles.  The single-CTA kernel,
@@ -952,7 +1011,7 @@ static int launch_gemm(const CUtensorMap &mA, const CUtensorMap &mB, const GemmA
 
 static size_t gemm2_smem_bytes(int H) {
   return 1024 + (size_t)STAGES2 * 2 * STAGE2_BYTES + (2 * STAGES2 + 5) * 8 + 16 +
-         (size_t)(epi_threads(H) - 64) * SCRATCH_F * sizeof(float);
+         CAND_BYTES;
 }
 
 // Epilogue halves of a launch of kernel `kind`: the CTA-pair kernel always
@@ -1316,6 +1375,7 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   const int lists_per_row = halves * g.splits;  // partial lists each row leaves
   g.num_kb = (eng->rdim + BK - 1) / BK;
   g.score_mode = eng->score_mode;
+  g.k = eng->k;
   g.mpad = g.num_m_tiles * tile;
   g.scaleB = eng->scaleB;
   g.part_vals = eng->part_vals;
@@ -1508,6 +1568,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   g.splits = splits;
   g.num_kb = (rdim + BK - 1) / BK;
   g.score_mode = score_mode;
+  g.k = k;
   g.mpad = (int)mpad;
   g.scaleB = d_scaleB;
   long long *pace = reinterpret_cast<long long *>(scratch);
