@@ -44,7 +44,7 @@ constexpr int A_STAGE = BM * BK;  // 16 KiB
 constexpr int B_STAGE = BN * BK;  // 32 KiB
 constexpr int TMEM_COLS = 512;
 constexpr long long WAIT_LIMIT = 4000000000LL;  // clock cycles (~2 s)
-constexpr int MAX_SPLITS = 128;
+constexpr int MAX_LISTS = 128;  // partial lists per row (column splits x epilogue halves)
 // Epilogue forms of both kernels: 4 * H epilogue warps.  With H = 2 two warps
 // share each TMEM lane quarter, each draining one half (128 columns) of
 // every tile into its own reservoir, so a (read tile, column split) unit
@@ -820,79 +820,119 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   }
 }
 
-// Merge the per-split sorted lists of every row into its final top-k:
-// one warp per row, k rounds of a warp arg-max over the list heads.
-__global__ void k_merge_splits(const float *__restrict__ pv, const int *__restrict__ pc, int splits,
-                               int mpad, int KT, int nb, int k, int score_mode,
-                               const float *__restrict__ scaleA, float *out_v, int *out_l) {
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (row >= nb) return;
-  const unsigned FULL = 0xFFFFFFFFu;
-  constexpr int PER = MAX_SPLITS / 32;
-  int head[PER];
-  float hv[PER];
-  int hc[PER];
+// Merge the per-split sorted lists of every row into its final top-k: G lanes
+// per row, PER lists per lane, k rounds of an arg-max over the list heads.
+// Each lane holds the next four entries of its lists in registers, so the
+// rounds run without touching memory until a list has given four of the k
+// (with one entry held, every round waited for the load of the winner's
+// successor: k L2 latencies, 16-20 us whatever the batch).  G follows the
+// number of lists, so that a row of a large batch (few lists) does not
+// occupy a whole warp: 65,536 rows of 4 lists 308 -> 44 us, 8,192 rows of 32
+// lists 39 -> 20, 16 to 200 rows of 128 lists 18 -> 12 (launch included).
+template <int G, int PER>
+__global__ void __launch_bounds__(256) k_merge_splits(const float *__restrict__ pv, const int *__restrict__ pc,
+                                                     int lists, int mpad, int KT, int nb, int k,
+                                                     const float *__restrict__ scaleA, float *out_v, int *out_l) {
+  const int gl = threadIdx.x % G;
+  const int row = blockIdx.x * (256 / G) + threadIdx.x / G;
+  if (row >= nb) return;  // whole groups
+  const unsigned gmask = G == 32 ? 0xFFFFFFFFu : ((1u << G) - 1u) << ((threadIdx.x & 31) / G * G);
+  float v[PER][4];
+  int c[PER][4], taken[PER];
 #pragma unroll
   for (int q = 0; q < PER; ++q) {
-    int s = lane + 32 * q;
-    head[q] = 0;
-    if (s < splits) {
-      size_t b = ((size_t)s * mpad + row) * KT;
-      hv[q] = pv[b];
-      hc[q] = pc[b];
-    } else {
-      hv[q] = -INFINITY;
-      hc[q] = INT_MAX;
+    const int s = gl + G * q;
+    float4 a = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    int4 b = make_int4(INT_MAX, INT_MAX, INT_MAX, INT_MAX);
+    if (s < lists) {
+      const size_t at = ((size_t)s * mpad + row) * KT;
+      a = *reinterpret_cast<const float4 *>(pv + at);
+      b = *reinterpret_cast<const int4 *>(pc + at);
     }
+    v[q][0] = a.x, v[q][1] = a.y, v[q][2] = a.z, v[q][3] = a.w;
+    c[q][0] = b.x, c[q][1] = b.y, c[q][2] = b.z, c[q][3] = b.w;
+    taken[q] = 0;
   }
-  const float sa = (score_mode == R2M_SCORE_SCALED) ? scaleA[row] : 1.0f;
+  const float sa = scaleA ? scaleA[row] : 1.0f;
   for (int r = 0; r < k; ++r) {
-    float bv = hv[0];
-    int bc = hc[0], bq = 0;
+    float bv = v[0][0];
+    int bc = c[0][0], bq = 0;
 #pragma unroll
     for (int q = 1; q < PER; ++q) {
-      bool better = (hv[q] > bv) || (hv[q] == bv && hc[q] < bc);
-      bv = better ? hv[q] : bv;
-      bc = better ? hc[q] : bc;
+      const bool better = v[q][0] > bv || (v[q][0] == bv && c[q][0] < bc);
+      bv = better ? v[q][0] : bv;
+      bc = better ? c[q][0] : bc;
       bq = better ? q : bq;
     }
-    float wv = bv;
-    int wc = bc, wl = lane;
+    // (value desc, column asc) as unsigned keys; -0 counts as +0
+    const uint32_t u = __float_as_uint(bv + 0.0f);
+    uint32_t key = (u >> 31) ? ~u : (u | 0x80000000u);
+    uint32_t col = (uint32_t)bc;
+    const uint32_t mykey = key;
+    if constexpr (G == 32) {
+      key = __reduce_max_sync(gmask, key);
+      col = __reduce_min_sync(gmask, mykey == key ? col : 0xFFFFFFFFu);
+    } else {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      float ov = __shfl_xor_sync(FULL, wv, o);
-      int oc = __shfl_xor_sync(FULL, wc, o);
-      int ol = __shfl_xor_sync(FULL, wl, o);
-      bool better = (ov > wv) || (ov == wv && oc < wc) || (ov == wv && oc == wc && ol < wl);
-      wv = better ? ov : wv;
-      wc = better ? oc : wc;
-      wl = better ? ol : wl;
+      for (int o = G / 2; o > 0; o >>= 1) {
+        const uint32_t ok = __shfl_xor_sync(gmask, key, o), oc = __shfl_xor_sync(gmask, col, o);
+        const bool better = ok > key || (ok == key && oc < col);
+        key = better ? ok : key;
+        col = better ? oc : col;
+      }
     }
-    if (lane == 0) {
-      bool empty = (wv == -INFINITY) || wc == INT_MAX;
-      out_v[(size_t)row * k + r] = empty ? -INFINITY : wv * sa;
-      out_l[(size_t)row * k + r] = empty ? 0 : wc + 1;
-    }
-    if (lane == wl) {
+    if (col == (uint32_t)INT_MAX) {  // every list is empty
+      if (gl == 0) {
+        out_v[(size_t)row * k + r] = -INFINITY;
+        out_l[(size_t)row * k + r] = 0;
+      }
+    } else if (mykey == key && (uint32_t)bc == col) {  // columns are distinct: one lane
+      out_v[(size_t)row * k + r] = bv * sa;
+      out_l[(size_t)row * k + r] = bc + 1;
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
-        if (q == bq) {
-          int s = lane + 32 * q;
-          int h = ++head[q];
-          if (h < KT) {
-            size_t b = ((size_t)s * mpad + row) * KT + h;
-            hv[q] = pv[b];
-            hc[q] = pc[b];
-          } else {
-            hv[q] = -INFINITY;
-            hc[q] = INT_MAX;
-          }
+        if (q != bq) continue;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          v[q][e] = v[q][e + 1];
+          c[q][e] = c[q][e + 1];
+        }
+        v[q][3] = -INFINITY;
+        c[q][3] = INT_MAX;
+        if ((++taken[q] & 3) == 0 && taken[q] < KT) {
+          const size_t at = ((size_t)(gl + G * q) * mpad + row) * KT + taken[q];
+          const float4 a = *reinterpret_cast<const float4 *>(pv + at);
+          const int4 b = *reinterpret_cast<const int4 *>(pc + at);
+          v[q][0] = a.x, v[q][1] = a.y, v[q][2] = a.z, v[q][3] = a.w;
+          c[q][0] = b.x, c[q][1] = b.y, c[q][2] = b.z, c[q][3] = b.w;
         }
       }
     }
-    __syncwarp();
+    __syncwarp(gmask);
   }
+}
+
+template <int G, int PER>
+static void launch_merge_as(const GemmArgs &g, int lists, int KT, const float *scaleA, float *vals, int *locs,
+                            cudaStream_t st) {
+  constexpr int rows = 256 / G;
+  k_merge_splits<G, PER><<<(g.nb + rows - 1) / rows, 256, 0, st>>>(g.part_vals, g.part_cols, lists, g.mpad, KT, g.nb,
+                                                                  g.k, scaleA, vals, locs);
+}
+
+// Merge the `lists` partial lists a launch with arguments g left per row.
+static int launch_merge(const GemmArgs &g, int lists, int KT, const float *scaleA, float *vals, int *locs,
+                        cudaStream_t st) {
+  static_assert(MAX_LISTS <= 32 * 4, "the widest merge holds 128 lists");
+  if (g.score_mode != R2M_SCORE_SCALED) scaleA = nullptr;
+  if (lists <= 4) launch_merge_as<4, 1>(g, lists, KT, scaleA, vals, locs, st);
+  else if (lists <= 8) launch_merge_as<8, 1>(g, lists, KT, scaleA, vals, locs, st);
+  else if (lists <= 16) launch_merge_as<8, 2>(g, lists, KT, scaleA, vals, locs, st);
+  else if (lists <= 32) launch_merge_as<32, 1>(g, lists, KT, scaleA, vals, locs, st);
+  else if (lists <= 64) launch_merge_as<32, 2>(g, lists, KT, scaleA, vals, locs, st);
+  else launch_merge_as<32, 4>(g, lists, KT, scaleA, vals, locs, st);
+  R2M_CUDA(cudaGetLastError());
+  return R2M_OK;
 }
 
 // ------------------------------------------------------------------ host
@@ -957,7 +997,7 @@ static size_t gemm_smem_bytes(int H) {
 // 16,384-65,536 reads: one split beat the imbalance-minimising choice by 8-18%
 // below 65,536 reads); so there the splits maximise
 // units / (waves x pairs) x 0.91^log2(splits) over 1..8.
-static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max_splits = MAX_SPLITS,
+static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max_splits = MAX_LISTS,
                          bool pair = false) {
   if (forced > 0) {
     int s = forced;
@@ -1075,7 +1115,12 @@ static int preload_kernels() {
 #undef R2M_PRELOAD1
 #undef R2M_PRELOAD2
   cudaFuncAttributes fa;
-  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<4, 1>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<8, 1>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<8, 2>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 1>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 2>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 4>));
   done[dev] = true;
   return R2M_OK;
 }
@@ -1148,7 +1193,7 @@ static size_t lists_needed(int rows_cap, int n_tiles, int ctas, int forced, int 
     // either kernel may leave two partial lists per row and split
     (void)kind;
     const int H = KT <= 32 ? 2 : 1;
-    size_t l = (size_t)choose_splits(mt, n_tiles, c, forced, MAX_SPLITS / H, kind == 2) * H * mt * tile;
+    size_t l = (size_t)choose_splits(mt, n_tiles, c, forced, MAX_LISTS / H, kind == 2) * H * mt * tile;
     if (l > lists) lists = l;
   }
   return lists;
@@ -1369,7 +1414,7 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.N = eng->N;
   g.n_tiles = eng->n_tiles;
   const int hmax = eng->KT <= 32 ? 2 : 1;
-  g.splits = choose_splits(g.num_m_tiles, eng->n_tiles, ctas_eff, eng->forced_splits, MAX_SPLITS / hmax, kind == 2);
+  g.splits = choose_splits(g.num_m_tiles, eng->n_tiles, ctas_eff, eng->forced_splits, MAX_LISTS / hmax, kind == 2);
   const int halves =
       eng->epi == 1 ? 1 : eng->epi == 2 ? hmax : epi_halves_for(kind, eng->KT, eng->n_tiles, g.splits);
   const int lists_per_row = halves * g.splits;  // partial lists each row leaves
@@ -1397,11 +1442,7 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   rc = dispatch_gemm(kind, halves, eng->KT, mapA, eng->mapB, eng->mapB128, g, ctas, st);
   if (rc) return rc;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[1], st));
-  const int warps = 8;
-  k_merge_splits<<<(nb + warps - 1) / warps, 32 * warps, 0, st>>>(
-      eng->part_vals, eng->part_cols, lists_per_row, g.mpad, eng->KT, nb, eng->k, eng->score_mode, d_scaleA,
-      d_vals, d_locs);
-  R2M_CUDA(cudaGetLastError());
+  if ((rc = launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, st))) return rc;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[2], st));
   return R2M_OK;
 }
@@ -1553,7 +1594,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   const int ctas_eff = kind == 2 ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
   const int hmax = KT <= 32 ? 2 : 1;
   // the engine's automatic schedule, with the splits cut to the scratch
-  int splits = choose_splits(m_tiles, n_tiles, ctas_eff, 0, MAX_SPLITS / hmax, kind == 2);
+  int splits = choose_splits(m_tiles, n_tiles, ctas_eff, 0, MAX_LISTS / hmax, kind == 2);
   int halves = epi_halves_for(kind, KT, n_tiles, splits);
   while (splits > 1 && (size_t)halves * splits * mpad > max_lists) {
     --splits;
@@ -1591,11 +1632,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   }
   rc = dispatch_gemm(kind, halves, KT, mapA, mapB, mapB128, g, ctas, st);
   if (rc) return rc;
-  const int warps = 8;
-  k_merge_splits<<<(nb + warps - 1) / warps, 32 * warps, 0, st>>>(g.part_vals, g.part_cols, halves * splits,
-                                                                   g.mpad, KT, nb, k, score_mode, d_scaleA,
-                                                                   d_vals, d_locs);
-  R2M_CUDA(cudaGetLastError());
+  if ((rc = launch_merge(g, halves * splits, KT, d_scaleA, d_vals, d_locs, st))) return rc;
   k_noalloc_poison<<<64, 256, 0, st>>>(err, d_vals, d_locs, (long long)nb * k);
   R2M_CUDA(cudaGetLastError());
   return R2M_OK;
