@@ -632,6 +632,18 @@ __device__ __forceinline__ uint32_t lanerev32(uint32_t x) {
   return (x << 16) | (x >> 16);
 }
 
+// Reverse complement of a fragment held one word per lane (lane t: word t,
+// zero for t >= W): complement, left-align the k bases to the end of the
+// W-word stream, reverse the word order and the sixteen 2-bit lanes.
+// shbits = 32 W - 2 k.  Called by the whole warp.
+__device__ __forceinline__ uint32_t revcomp_reg(uint32_t w, int W, uint32_t shbits) {
+  const int lane = threadIdx.x & 31, src = W - 1 - lane;
+  const uint32_t xi = ~__shfl_sync(0xFFFFFFFFu, w, src & 31), xm = ~__shfl_sync(0xFFFFFFFFu, w, (src - 1) & 31);
+  uint32_t v = xi;
+  if (shbits != 0) v = (xi << shbits) | (src > 0 ? (xm >> (32u - shbits)) : 0u);
+  return lane < W ? lanerev32(v) : 0u;
+}
+
 // One thread per output word: complement, left-align the k bases to the end
 // of the W-word stream, then reverse word order and the sixteen 2-bit lanes.
 __global__ void k_revcomp(uint32_t *drc, const uint32_t *dnas, int W, int64_t n, uint32_t shbits) {
@@ -1035,7 +1047,6 @@ __global__ void __launch_bounds__(256, M <= 4 ? 4 : 1) k_encode_sparse_ref(EncPa
   float2 *table = reinterpret_cast<float2 *>(smem);
   sparse_table(P, table);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned FULL = 0xFFFFFFFFu;
   const SparseLayout L = sparse_layout(P.c, M, P.sp_nslot, OutT<OUT>::bytes);
   unsigned char *warea = smem + sparse_table_bytes(P) + (size_t)L.warp * warp;
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -1052,13 +1063,7 @@ __global__ void __launch_bounds__(256, M <= 4 ? 4 : 1) k_encode_sparse_ref(EncPa
       fw = __funnelshift_r(a, b, (uint32_t)(pos & 15) << 1);
       if (lane == P.W - 1) fw &= tailmask;
     }
-    // reverse complement: complement, left-align the k bases to the end of
-    // the W-word stream, reverse the word order and the sixteen 2-bit lanes
-    const int src = P.W - 1 - lane;
-    const uint32_t xi = ~__shfl_sync(FULL, fw, src & 31), xm = ~__shfl_sync(FULL, fw, (src - 1) & 31);
-    uint32_t vv = xi;
-    if (shbits != 0) vv = (xi << shbits) | (src > 0 ? (xm >> (32u - shbits)) : 0u);
-    const uint32_t rcw = lane < P.W ? lanerev32(vv) : 0u;
+    const uint32_t rcw = revcomp_reg(fw, P.W, shbits);
     const int64_t bt = i / batch, off = i - bt * batch;
     const int64_t nb = min(batch, nwin - bt * batch);
     const int64_t colf = 2 * bt * batch + off, colr = colf + nb;
@@ -1476,6 +1481,214 @@ __global__ void __launch_bounds__(128) k_rescore_fp32(EncParams P, const uint32_
   }
 }
 
+// The same for the encoders in use (normalize = 0, m = 1, 2 or 4, 256, 512 or
+// 1024 bins, fragments of at most 496 bases): one block of four warps per
+// read, the candidates dealt out to its warps.  What bounds it is instruction
+// issue: a candidate is a whole encode (nw windows) and a dot product over
+// every bin, against a few hundred bytes of memory traffic.  So
+//   * a lane's 2T embedding values of the read (bins lane + 32 t) stay in its
+//     registers for all candidates;
+//   * the dot product divides with the encoder's reciprocal + FMA correction
+//     (the correctly rounded x / nrm) on (Re, Im) pairs;
+//   * window groups come from shared lane masks and are added in rounds, as
+//     in sparse_fragment, but into the dense histogram, whose linear passes
+//     cost less here than slots looked up per bin;
+//   * the ranks of the candidates are counted by all lanes.
+// 4,000 reads x 64 candidates of 150 bases (s8 m4 c4): 3,900 us with the general
+// kernel, 774 us with this one.
+// Every sum is formed in the general kernel's order (bins in window order, the
+// energies along float4 slots, the dot product over bins lane + 32 t, Re
+// before Im), so the scores are the same bits.
+template <int M, int T>
+__device__ __forceinline__ float rescore_hist(const EncParams &P, const float2 *__restrict__ table, float *hist,
+                                              uint32_t *gmask, uint32_t wreg) {
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xFFFFFFFFu;
+  const unsigned lt = (1u << lane) - 1u;
+  float4 *h4 = reinterpret_cast<float4 *>(hist);
+#pragma unroll
+  for (int i = 0; i < T / 2; ++i) h4[lane + 32 * i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  __syncwarp();
+  const int nw = P.nw;
+  const uint32_t bmask = P.bmask, cbmask = P.cbmask, c2 = 2u * (uint32_t)P.c;
+  for (int b0 = 0; b0 < nw; b0 += 32) {
+    const int p = b0 + lane;
+    const bool valid = p < nw;
+    const int wo = p >> 4;
+    const uint32_t w0 = __shfl_sync(FULL, wreg, wo & 31), w1 = __shfl_sync(FULL, wreg, (wo + 1) & 31);
+    const uint32_t smer = __funnelshift_r(w0, w1, (uint32_t)(p & 15) << 1) & bmask;
+    const uint32_t upper = c2 >= 32u ? 0u : (smer >> c2);
+    const uint32_t cb = (smer & cbmask) ^ ((upper * 0x9E3779B1u) & cbmask);
+    if (valid) atomicOr(gmask + cb, 1u << lane);
+    __syncwarp();
+    const unsigned grp = valid ? gmask[cb] : (1u << lane);
+    const int rank = __popc(grp & lt);
+    const int rounds = (int)__reduce_max_sync(FULL, (unsigned)rank);
+    float2 ph[M];
+    if (valid) ld_planes<M>(table, nw, p, ph);
+    __syncwarp();
+    if (valid && rank == 0) gmask[cb] = 0u;
+    for (int r = 0; r <= rounds; ++r) {
+      if (valid && rank == r) {
+        if constexpr (M == 1) {
+          float2 *h = reinterpret_cast<float2 *>(hist + hoff((int)cb));
+          *h = add2(*h, ph[0]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < M / 2; ++q) {
+            float4 *h = reinterpret_cast<float4 *>(hist + hoff((int)(cb * M + 2 * q)));
+            const float4 t = *h;
+            const float2 a = add2(make_float2(t.x, t.y), ph[2 * q]), b = add2(make_float2(t.z, t.w), ph[2 * q + 1]);
+            *h = make_float4(a.x, a.y, b.x, b.y);
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  if (lane < M) *reinterpret_cast<float2 *>(hist + hoff((int)(P.csmerG * M + lane))) = make_float2(0.f, 0.f);
+  __syncwarp();
+  // energies along the float4 slots, as fragment_hist takes them
+  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+  for (int i = 0; i < T / 2; ++i) {
+    const float4 t = h4[lane + 32 * i];
+    const float e0 = __fadd_rn(__fmul_rn(t.x, t.x), __fmul_rn(t.y, t.y));
+    const float e1 = __fadd_rn(__fmul_rn(t.z, t.z), __fmul_rn(t.w, t.w));
+    const bool hi = (((lane & 7) ^ (((lane >> 3) + 4 * i) & 7)) & 1) != 0;
+    if (hi) {
+      a2 += e0;
+      a3 += e1;
+    } else {
+      a0 += e0;
+      a1 += e1;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    a0 += __shfl_xor_sync(FULL, a0, o);
+    a1 += __shfl_xor_sync(FULL, a1, o);
+    a2 += __shfl_xor_sync(FULL, a2, o);
+    a3 += __shfl_xor_sync(FULL, a3, o);
+  }
+  float tot;
+  if constexpr (M == 4) tot = ((a0 + a1) + a2) + a3;
+  else if constexpr (M == 2) tot = (a0 + a2) + (a1 + a3);
+  else tot = (a0 + a2) + (a1 + a3);
+  return (float)((double)sqrtf(tot) + 1e-16);
+}
+
+constexpr int kRescoreWarps = 4;
+
+template <int M, int T>
+__global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
+    EncParams P, const uint32_t *__restrict__ dnas, int nb, const int *__restrict__ cand, int kc,
+    const uint32_t *__restrict__ genome, const int64_t *__restrict__ col_pos, const uint8_t *__restrict__ strand,
+    long long N, float *scores, float *out_v, int *out_l, int k) {
+  constexpr int NCM = 32 * T / M;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ float sc[kMaxCand];
+  __shared__ int scol[kMaxCand];
+  float2 *table = reinterpret_cast<float2 *>(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned FULL = 0xFFFFFFFFu;
+  float *hist = reinterpret_cast<float *>(smem + sparse_table_bytes(P)) + warp * (64 * T + NCM);
+  uint32_t *gmask = reinterpret_cast<uint32_t *>(hist + 64 * T);
+  for (int i = lane; i < NCM; i += 32) gmask[i] = 0u;
+  sparse_table(P, table);  // ends with a block barrier
+  const int W = P.W, rr = P.k & 15;
+  const uint32_t tailmask = rr == 0 ? 0xFFFFFFFFu : ((1u << (2 * rr)) - 1u);
+  const uint32_t shbits = (uint32_t)(32 * W - 2 * P.k);
+  for (int row = blockIdx.x; row < nb; row += gridDim.x) {
+    // the read's embedding: values of bins lane + 32 t
+    float2 emb[T];
+    {
+      const uint32_t wreg = lane < W ? __ldg(dnas + (size_t)row * W + lane) : 0u;
+      const float nrm = rescore_hist<M, T>(P, table, hist, gmask, wreg);
+      const float y = __frcp_rn(nrm);
+      const float2 y2 = make_float2(y, y), nn2 = make_float2(-nrm, -nrm);
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const float2 x = *reinterpret_cast<const float2 *>(hist + hoff(lane + 32 * t));
+        const float2 q0 = mul2(x, y2);
+        emb[t] = fma2(fma2(q0, nn2, x), y2, q0);
+      }
+      __syncwarp();
+    }
+    for (int j = warp; j < kc; j += kRescoreWarps) {
+      const int c1 = __ldg(cand + (size_t)row * kc + j);
+      float s = -INFINITY;
+      if (c1 >= 1 && c1 <= N) {
+        const long long col = c1 - 1;
+        const int64_t pos = __ldg(col_pos + col);
+        const int64_t q = pos >> 4;
+        uint32_t wreg = 0u;
+        if (lane < W) {
+          const uint32_t a = __ldg(genome + q + lane), b = __ldg(genome + q + lane + 1);
+          wreg = __funnelshift_r(a, b, (uint32_t)(pos & 15) << 1);
+          if (lane == W - 1) wreg &= tailmask;
+        }
+        if (__ldg(strand + col)) wreg = revcomp_reg(wreg, W, shbits);
+        const float nrm = rescore_hist<M, T>(P, table, hist, gmask, wreg);
+        const float y = __frcp_rn(nrm);
+        float acc = 0.f;
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          const float x = hist[hoff(lane + 32 * t)], q0 = x * y;
+          acc = fmaf(emb[t].x, fmaf(fmaf(-q0, nrm, x), y, q0), acc);
+        }
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          const float x = hist[hoff(lane + 32 * t) + 1], q0 = x * y;
+          acc = fmaf(emb[t].y, fmaf(fmaf(-q0, nrm, x), y, q0), acc);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+        s = acc;
+        __syncwarp();
+      }
+      if (lane == 0) {
+        sc[j] = s;
+        scol[j] = c1;
+        if (scores) scores[(size_t)row * kc + j] = s;
+      }
+    }
+    __syncthreads();
+    // rank of each candidate: score descending, column ascending
+    if (threadIdx.x < kc) {
+      const float v = sc[threadIdx.x];
+      const int c = scol[threadIdx.x];
+      int rank = 0;
+      for (int j = 0; j < kc; ++j) {
+        const float ov = sc[j];
+        const int oc = scol[j];
+        rank += (ov > v || (ov == v && (oc < c || (oc == c && j < (int)threadIdx.x)))) ? 1 : 0;
+      }
+      if (rank < k) {
+        out_v[(size_t)row * k + rank] = v;
+        out_l[(size_t)row * k + rank] = v == -INFINITY ? 0 : c;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int M, int T>
+static int launch_rescore(const EncParams &P, const uint32_t *dnas, int nb, const int *cand, int kc,
+                          const uint32_t *genome, const int64_t *col_pos, const uint8_t *strand, long long N,
+                          float *scores, float *out_v, int *out_l, int k, cudaStream_t st) {
+  auto kern = k_rescore_dense<M, T>;
+  const size_t smem = sparse_table_bytes(P) + (size_t)kRescoreWarps * (64 * T + 32 * T / M) * 4;
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 1;
+  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kRescoreWarps, smem));
+  const long long cap = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
+  kern<<<(unsigned)(nb < cap ? nb : cap), 32 * kRescoreWarps, smem, st>>>(P, dnas, nb, cand, kc, genome, col_pos,
+                                                                         strand, N, scores, out_v, out_l, k);
+  R2M_CUDA(cudaGetLastError());
+  return R2M_OK;
+}
+
 }  // namespace r2m
 
 extern "C" int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *cand, int kc,
@@ -1491,6 +1704,19 @@ extern "C" int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *can
   if (nb == 0) return R2M_OK;
   R2M_REQUIRE(dnas && cand && genome && col_pos && strand && out_vals && out_locs, "null pointer");
   cudaStream_t st = as_stream(stream);
+  const char *force = getenv("R2M_ENCODER");
+  if (P.normalize == 0 && P.W <= 31 && !(force && strcmp(force, "dense") == 0)) {
+#define R2M_RESCORE(M_, T_)                                                                                    \
+  if (P.m == M_ && P.nbin == 32 * T_)                                                                          \
+  return launch_rescore<M_, T_>(P, dnas, nb, cand, kc, genome, col_pos, strand, N, scores, out_vals, out_locs, \
+                                topk, st)
+    R2M_RESCORE(4, 32);
+    R2M_RESCORE(4, 8);
+    R2M_RESCORE(2, 16);
+    R2M_RESCORE(1, 32);
+    R2M_RESCORE(1, 8);
+#undef R2M_RESCORE
+  }
   size_t tb = ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
   size_t per = warp_bytes_host(P) + (size_t)P.rdim * 4 + 2 * kMaxCand * 4 + 32;
   P.table_in_smem = (tb + per * 4 <= 200 * 1024) ? 1 : 0;
