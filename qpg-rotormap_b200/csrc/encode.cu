@@ -28,6 +28,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <cmath>
+
 #include "common.cuh"
 
 namespace r2m {
@@ -104,7 +106,7 @@ __device__ __forceinline__ float2 ref_phasor(const EncParams &P, int idm, int p)
 
 // Global table (used when the per-block shared copy does not fit):
 // one thread per (idm, reference chunk) walks the chunk's recurrence.
-__global__ void k_phasor_table(EncParams P, float2 *table) {
+__global__ void k_phasor_table(EncParams P, int pitch, float2 *table) {
   int nchunk = (P.nw + P.Wc - 1) / P.Wc;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nchunk * P.m) return;
@@ -115,7 +117,7 @@ __global__ void k_phasor_table(EncParams P, float2 *table) {
   float re = cosf(a), im = sinf(a);
   float xr = cosf(th), xi = sinf(th);
   for (int p = p0; p < p1; ++p) {
-    table[(size_t)idm * P.nw + p] = make_float2(re, im);
+    table[(size_t)idm * pitch + p] = make_float2(re, im);
     float nr = __fsub_rn(__fmul_rn(re, xr), __fmul_rn(im, xi));
     float ni = __fadd_rn(__fmul_rn(re, xi), __fmul_rn(im, xr));
     re = nr;
@@ -216,80 +218,14 @@ __device__ __forceinline__ float out_value(const EncParams &P, const float *hist
   return x;
 }
 
-// Histogram of the fragment whose words are staged in `words` (W words + a
-// zero guard word), built by one warp: phasor sums per bin in window order,
-// G-homopolymer bins zeroed, modes 2/3 reshaped; `nrmv` receives the divisor
-// of every copy (index 0 for mode 0) and `norms_out` the reference's norms
-// row.  The normalised value of split element i is hist[...]/nrmv[...].
-__device__ __forceinline__ void fragment_hist(const EncParams &P, const float2 *table, float *hist, uint16_t *cs,
-                              const uint32_t *words, float *nrmv, float *norms_out, float *amax_raw = nullptr) {
+// The rest of a fragment's histogram once its windows are summed, by one
+// warp: G-homopolymer bins zeroed, modes 2/3 reshaped; `nrmv` receives the
+// divisor of every copy (index 0 for mode 0) and `norms_out` the reference's
+// norms row.  The normalised value of split element i is hist[...]/nrmv[...].
+__device__ __forceinline__ void finish_hist(const EncParams &P, float *hist, float *nrmv, float *norms_out,
+                                            float *amax_raw) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
-  // zero the histogram
-  for (int i = lane * 4; i < P.hist_floats; i += 128)
-    *reinterpret_cast<float4 *>(hist + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-  // scrambled c-mer of every window
-  for (int p = lane; p < P.nw; p += 32) {
-    int wo = p >> 4;
-    uint32_t sh = (uint32_t)(p & 15) << 1;
-    uint32_t w0 = words[wo], w1 = words[wo + 1];
-    uint32_t v = sh == 0 ? w0 : ((w0 >> sh) | (w1 << (32u - sh)));
-    uint32_t smer = v & P.bmask;
-    uint32_t lower = smer & P.cbmask;
-    uint32_t upper = (2 * P.c >= 32) ? 0u : (smer >> (2 * P.c));
-    uint32_t key = (upper * 0x9E3779B1u) & P.cbmask;
-    cs[p] = (uint16_t)(lower ^ key);
-  }
-  __syncwarp();
-  // accumulate phasors in increasing window order (deterministic)
-  for (int b0 = 0; b0 < P.nw; b0 += 32) {
-    int p = b0 + lane;
-    bool act = p < P.nw;
-    unsigned amask = __ballot_sync(FULL, act);
-    if (act) {
-      uint32_t cbin = cs[p];
-      unsigned grp = __match_any_sync(amask, cbin);
-      if (lane == __ffs(grp) - 1) {
-        if (P.m == 4) {
-          // the group's bins 4 cbin .. 4 cbin + 3 (float4 slots 2 (cbin % 4)
-          // and the next one of chunk cbin / 4, swizzled): one read-modify-
-          // write, the members' phasors added in window (lane) order
-          float4 *hc = reinterpret_cast<float4 *>(hist + ((cbin >> 2) << 5));
-          const int sw = (int)((cbin >> 2) & 7), s0 = (int)(2 * (cbin & 3));
-          float4 *h0 = hc + (s0 ^ sw), *h1 = hc + ((s0 + 1) ^ sw);
-          float4 h01 = *h0, h23 = *h1;
-          unsigned g = grp;
-          do {
-            const int j = __ffs(g) - 1;
-            g &= g - 1;
-            const float2 p0 = table[b0 + j], p1 = table[(size_t)P.nw + b0 + j];
-            const float2 p2 = table[2 * (size_t)P.nw + b0 + j], p3 = table[3 * (size_t)P.nw + b0 + j];
-            h01.x += p0.x; h01.y += p0.y; h01.z += p1.x; h01.w += p1.y;
-            h23.x += p2.x; h23.y += p2.y; h23.z += p3.x; h23.w += p3.y;
-          } while (g);
-          *h0 = h01;
-          *h1 = h23;
-        } else {
-          for (int idm = 0; idm < P.m; ++idm) {
-            float *h = hist + hoff((int)(cbin * P.m + idm));
-            float re = h[0], im = h[1];
-            const float2 *tb = table + (size_t)idm * P.nw + b0;
-            unsigned g = grp;
-            while (g) {
-              int j = __ffs(g) - 1;
-              g &= g - 1;
-              float2 ph = tb[j];
-              re += ph.x;
-              im += ph.y;
-            }
-            h[0] = re;
-            h[1] = im;
-          }
-        }
-      }
-    }
-    __syncwarp();
-  }
   // zero the G-homopolymer bins
   if (lane < P.m) {
     float *h = hist + hoff(P.csmerG * P.m + lane);
@@ -413,19 +349,92 @@ __device__ __forceinline__ void fragment_hist(const EncParams &P, const float2 *
   __syncwarp();
 }
 
-// Encode the fragment whose words are staged in `words` (W words + a zero
-// guard word) with one warp; write row `row` (rdim elements of OUT), the m
-// norms and (scaled e4m3) the row scale.
-template <int OUT>
-__device__ void encode_fragment(const EncParams &P, const float2 *table, float *hist,
-                                uint16_t *cs, const uint32_t *words, float *nrmv, void *row,
-                                float *norms_out, float *scale_out) {
+// Histogram of the fragment whose words are staged in `words` (W words + a
+// zero guard word), built and finished by one warp: phasor sums per bin in
+// window order.
+__device__ __forceinline__ void fragment_hist(const EncParams &P, const float2 *table, float *hist, uint16_t *cs,
+                              const uint32_t *words, float *nrmv, float *norms_out, float *amax_raw = nullptr) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
-  const bool fast = P.normalize == 0 && (P.nbin % 16) == 0 && P.nbin >= 16;
-  float amax_raw = 0.f;
-  fragment_hist(P, table, hist, cs, words, nrmv, norms_out, fast ? &amax_raw : nullptr);
-  if (fast) {
+  // zero the histogram
+  for (int i = lane * 4; i < P.hist_floats; i += 128)
+    *reinterpret_cast<float4 *>(hist + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+  // scrambled c-mer of every window
+  for (int p = lane; p < P.nw; p += 32) {
+    int wo = p >> 4;
+    uint32_t sh = (uint32_t)(p & 15) << 1;
+    uint32_t w0 = words[wo], w1 = words[wo + 1];
+    uint32_t v = sh == 0 ? w0 : ((w0 >> sh) | (w1 << (32u - sh)));
+    uint32_t smer = v & P.bmask;
+    uint32_t lower = smer & P.cbmask;
+    uint32_t upper = (2 * P.c >= 32) ? 0u : (smer >> (2 * P.c));
+    uint32_t key = (upper * 0x9E3779B1u) & P.cbmask;
+    cs[p] = (uint16_t)(lower ^ key);
+  }
+  __syncwarp();
+  // accumulate phasors in increasing window order (deterministic)
+  for (int b0 = 0; b0 < P.nw; b0 += 32) {
+    int p = b0 + lane;
+    bool act = p < P.nw;
+    unsigned amask = __ballot_sync(FULL, act);
+    if (act) {
+      uint32_t cbin = cs[p];
+      unsigned grp = __match_any_sync(amask, cbin);
+      if (lane == __ffs(grp) - 1) {
+        if (P.m == 4) {
+          // the group's bins 4 cbin .. 4 cbin + 3 (float4 slots 2 (cbin % 4)
+          // and the next one of chunk cbin / 4, swizzled): one read-modify-
+          // write, the members' phasors added in window (lane) order
+          float4 *hc = reinterpret_cast<float4 *>(hist + ((cbin >> 2) << 5));
+          const int sw = (int)((cbin >> 2) & 7), s0 = (int)(2 * (cbin & 3));
+          float4 *h0 = hc + (s0 ^ sw), *h1 = hc + ((s0 + 1) ^ sw);
+          float4 h01 = *h0, h23 = *h1;
+          unsigned g = grp;
+          do {
+            const int j = __ffs(g) - 1;
+            g &= g - 1;
+            const float2 p0 = table[b0 + j], p1 = table[(size_t)P.nw + b0 + j];
+            const float2 p2 = table[2 * (size_t)P.nw + b0 + j], p3 = table[3 * (size_t)P.nw + b0 + j];
+            h01.x += p0.x; h01.y += p0.y; h01.z += p1.x; h01.w += p1.y;
+            h23.x += p2.x; h23.y += p2.y; h23.z += p3.x; h23.w += p3.y;
+          } while (g);
+          *h0 = h01;
+          *h1 = h23;
+        } else {
+          for (int idm = 0; idm < P.m; ++idm) {
+            float *h = hist + hoff((int)(cbin * P.m + idm));
+            float re = h[0], im = h[1];
+            const float2 *tb = table + (size_t)idm * P.nw + b0;
+            unsigned g = grp;
+            while (g) {
+              int j = __ffs(g) - 1;
+              g &= g - 1;
+              float2 ph = tb[j];
+              re += ph.x;
+              im += ph.y;
+            }
+            h[0] = re;
+            h[1] = im;
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+  finish_hist(P, hist, nrmv, norms_out, amax_raw);
+}
+
+__device__ __forceinline__ bool fast_rows(const EncParams &P) {
+  return P.normalize == 0 && (P.nbin % 16) == 0 && P.nbin >= 16;
+}
+
+// Write a finished histogram as row `row` (rdim elements of OUT) and (scaled
+// e4m3) its scale.  Called by threads t of nt; nt = 32, one warp, unless
+// fast_rows(P), which needs amax_raw from finish_hist.
+template <int OUT>
+__device__ __forceinline__ void write_row(const EncParams &P, const float *hist, const float *nrmv, float amax_raw,
+                                          void *row, float *scale_out, int t, int nt) {
+  if (fast_rows(P)) {
     // one output pass: each lane takes chunks of 16 bins, divides every value
     // by the norm, scales, converts and stores the chunk's Re and Im runs
     const float nrm = nrmv[0];
@@ -445,19 +454,19 @@ __device__ void encode_fragment(const EncParams &P, const float2 *table, float *
       // normalised magnitude is the largest raw magnitude divided once
       const float amax = divn(amax_raw);
       scale = amax > 0.f ? 448.0f / amax : 1.0f;
-      if (lane == 0) *scale_out = amax > 0.f ? amax / 448.0f : 0.0f;
+      if (t == 0) *scale_out = amax > 0.f ? amax / 448.0f : 0.0f;
     }
-    for (int j = lane; j < nchunk; j += 32) {
+    for (int j = t; j < nchunk; j += nt) {
       const float4 *h4 = reinterpret_cast<const float4 *>(hist + 32 * j);
       const int sw = j & 7;
       float re[16], im[16];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        float4 t = h4[q ^ sw];
-        re[2 * q] = divn(t.x);
-        im[2 * q] = divn(t.y);
-        re[2 * q + 1] = divn(t.z);
-        im[2 * q + 1] = divn(t.w);
+        const float4 z = h4[q ^ sw];
+        re[2 * q] = divn(z.x);
+        im[2 * q] = divn(z.y);
+        re[2 * q + 1] = divn(z.z);
+        im[2 * q + 1] = divn(z.w);
       }
       if constexpr (OUT == R2M_OUT_E4M3_SCALED) {
 #pragma unroll
@@ -474,9 +483,10 @@ __device__ void encode_fragment(const EncParams &P, const float2 *table, float *
         store16<OUT>(row, P.nbin + 16 * j, im);
       }
     }
-    __syncwarp();
     return;
   }
+  const int lane = t;
+  const unsigned FULL = 0xFFFFFFFFu;
   // output pass (amax first for the scaled form)
   float scale = 1.0f;
   if constexpr (OUT == R2M_OUT_E4M3_SCALED) {
@@ -486,7 +496,7 @@ __device__ void encode_fragment(const EncParams &P, const float2 *table, float *
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(FULL, amax, o));
     scale = amax > 0.f ? 448.0f / amax : 1.0f;
-    if (lane == 0) *scale_out = amax > 0.f ? amax / 448.0f : 0.0f;
+    if (t == 0) *scale_out = amax > 0.f ? amax / 448.0f : 0.0f;
   }
   const bool vec = (P.rdim % 16) == 0;
   if (vec) {
@@ -499,6 +509,18 @@ __device__ void encode_fragment(const EncParams &P, const float2 *table, float *
   } else {
     for (int i = lane; i < P.rdim; i += 32) store1<OUT>(row, i, out_value<OUT>(P, hist, nrmv, i, scale));
   }
+}
+
+// Encode the fragment whose words are staged in `words` (W words + a zero
+// guard word) with one warp; write row `row` (rdim elements of OUT), the m
+// norms and (scaled e4m3) the row scale.
+template <int OUT>
+__device__ void encode_fragment(const EncParams &P, const float2 *table, float *hist,
+                                uint16_t *cs, const uint32_t *words, float *nrmv, void *row,
+                                float *norms_out, float *scale_out) {
+  float amax_raw = 0.f;
+  fragment_hist(P, table, hist, cs, words, nrmv, norms_out, fast_rows(P) ? &amax_raw : nullptr);
+  write_row<OUT>(P, hist, nrmv, amax_raw, row, scale_out, threadIdx.x & 31, 32);
   __syncwarp();
 }
 
@@ -1074,6 +1096,247 @@ __global__ void __launch_bounds__(256, M <= 4 ? 4 : 1) k_encode_sparse_ref(EncPa
   }
 }
 
+// ------------------------------------------------------------------
+// Long fragments: one block per fragment.
+//
+// A 20,000 base fragment has 625 batches of 32 windows.  One warp walks them
+// one after another, each a chain of shared-memory steps, and a thousand such
+// fragments leave the SMs seven warps each.  The bins' sums have to be formed in
+// window order (so that rows are the same bytes whichever path made them), but
+// different bins' sums are independent: so the windows are sorted by c-mer, a
+// tile of TW windows at a time (a stable counting sort: every warp ranks its
+// own run of consecutive windows, and a scan over bins and warps gives each its
+// place), and then every thread sums one bin's windows of the tile in
+// order, from the tile's phasors in shared memory.  Bins keep their
+// running sums in the dense histogram, whose norms and output pass are
+// those of the one-warp path.  Counts are 16-bit pairs: TW < 65536.
+// What bounds it is issue (63% of cycles, 120,000 warp instructions per 20,000
+// bases).  1,000 fragments of 20,000 bases, s5 m1 c5: 1,657 -> 213 us; s8 m4 c4:
+// 1,765 -> 394 us.
+constexpr int kLongWarps = 16;
+constexpr int kLongThreads = 32 * kLongWarps;
+constexpr int kLongHash = 256;  // lane masks per warp (c-mers that share one are told apart by shuffles)
+
+struct LongLayout {
+  int order, counts, start, masks, hist, words, misc, total;  // byte offsets (the phasor tile at 0), total bytes
+};
+
+__host__ __device__ inline LongLayout long_layout(const EncParams &P, int TW) {
+  const int ncm = 1 << (2 * P.c);
+  LongLayout L;
+  L.order = P.m * TW * 8;
+  L.counts = L.order + TW * 2;
+  L.start = L.counts + kLongWarps * ncm * 2;
+  L.masks = L.start + ((ncm * 2 + 2 + 15) & ~15);
+  L.hist = L.masks + kLongWarps * kLongHash * 4;
+  L.words = L.hist + P.hist_floats * 4;
+  L.misc = L.words + P.words_u32 * 4;
+  L.total = L.misc + 32 + 4 * kLongWarps + 16;
+  return L;
+}
+
+// Word j of the fragment that starts at base `pos` of the packed genome.
+__device__ __forceinline__ uint32_t genome_word(const EncParams &P, const uint32_t *__restrict__ genome, int64_t pos,
+                                                int j) {
+  const int64_t q = (pos >> 4) + j;
+  uint32_t v = __funnelshift_r(__ldg(genome + q), __ldg(genome + q + 1), (uint32_t)(pos & 15) << 1);
+  const int r = P.k & 15;
+  if (j == P.W - 1 && r != 0) v &= (1u << (2 * r)) - 1u;
+  return v;
+}
+
+// Item i: fragment i of `src`, or (REF) column i of the index batches over the
+// windows win_pos of the packed genome `src`, the windows' forward columns
+// before their reverse complements within a batch.
+template <int OUT, int TW, bool REF>
+__global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
+                                                             const int64_t *__restrict__ win_pos, int64_t nwin,
+                                                             int64_t batch, int64_t items, void *dest, float *norms,
+                                                             float *scales, const float2 *__restrict__ gtable,
+                                                             int pitch) {
+  constexpr int CW = TW / kLongWarps, NB = CW / 32;  // windows and batches per warp and tile
+  extern __shared__ __align__(16) unsigned char smem[];
+  const LongLayout L = long_layout(P, TW);
+  float2 *tab = reinterpret_cast<float2 *>(smem);
+  uint16_t *order = reinterpret_cast<uint16_t *>(smem + L.order);
+  uint16_t *counts = reinterpret_cast<uint16_t *>(smem + L.counts);
+  uint16_t *start = reinterpret_cast<uint16_t *>(smem + L.start);
+  uint32_t *masks = reinterpret_cast<uint32_t *>(smem + L.masks);
+  float *hist = reinterpret_cast<float *>(smem + L.hist);
+  uint32_t *words = reinterpret_cast<uint32_t *>(smem + L.words);
+  float *nrmv = reinterpret_cast<float *>(smem + L.misc);
+  int *wsum = reinterpret_cast<int *>(smem + L.misc + 32);
+  float *amax_s = reinterpret_cast<float *>(wsum + kLongWarps);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned FULL = 0xFFFFFFFFu, lt = (1u << lane) - 1u;
+  const int ncm = 1 << (2 * P.c), npair = ncm >> 1;
+  const size_t rowbytes = (size_t)P.rdim * OutT<OUT>::bytes;
+  for (int i = tid; i < kLongWarps * kLongHash; i += kLongThreads) masks[i] = 0u;  // zero between batches
+  for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    if constexpr (REF) {
+      const int64_t b = it / (2 * batch), off = it - 2 * b * batch;
+      const int64_t nb = min(batch, nwin - b * batch);
+      const bool rc = off >= nb;
+      const int64_t pos = __ldg(win_pos + b * batch + (rc ? off - nb : off));
+      const uint32_t shbits = (uint32_t)(32 * P.W - 2 * P.k);
+      for (int j = tid; j < P.W; j += kLongThreads) {
+        uint32_t v;
+        if (!rc) {
+          v = genome_word(P, src, pos, j);
+        } else {  // complement, left-align to the end of the word stream, reverse words and lanes
+          const int i = P.W - 1 - j;
+          v = ~genome_word(P, src, pos, i);
+          if (shbits != 0) v = (v << shbits) | (i > 0 ? (~genome_word(P, src, pos, i - 1)) >> (32u - shbits) : 0u);
+          v = lanerev32(v);
+        }
+        words[j] = v;
+      }
+    } else {
+      for (int j = tid; j < P.W; j += kLongThreads) words[j] = __ldg(src + it * P.W + j);
+    }
+    if (tid == 0) words[P.W] = 0u;
+    for (int i = tid * 4; i < P.hist_floats; i += 4 * kLongThreads)
+      *reinterpret_cast<float4 *>(hist + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t0 = 0; t0 < P.nw; t0 += TW) {
+      // the tile's phasors, in flight during the sort
+      const int nt = min(TW, P.nw - t0), nt2 = (nt + 1) >> 1;
+      for (int idm = 0; idm < P.m; ++idm) {
+        const float2 *g = gtable + (size_t)idm * pitch + t0;
+        for (int i = tid; i < nt2; i += kLongThreads)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tab + idm * TW + 2 * i)),
+                       "l"(g + 2 * i)
+                       : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      uint32_t *c32 = reinterpret_cast<uint32_t *>(counts);
+      for (int i = tid; i < kLongWarps * npair; i += kLongThreads) c32[i] = 0u;
+      __syncthreads();
+      // rank of every window among its warp's windows of the same c-mer: the
+      // lanes of a batch find each other by OR-ing their bit into their
+      // c-mer's mask (__match_any_sync costs several times the rest of the tile)
+      uint32_t cbr[NB];  // c-mer, later | rank << 16
+      uint16_t *mine = counts + warp * ncm;
+      uint32_t *mask = masks + warp * kLongHash;
+      const int w0 = warp * CW + lane;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const int p = t0 + w0 + 32 * b, wo = w0 + 32 * b < nt ? p >> 4 : 0;
+        const uint32_t v = __funnelshift_r(words[wo], words[wo + 1], (uint32_t)(p & 15) << 1);
+        const uint32_t smer = v & P.bmask;
+        const uint32_t upper = (2 * P.c >= 32) ? 0u : (smer >> (2 * P.c));
+        cbr[b] = (smer & P.cbmask) ^ ((upper * 0x9E3779B1u) & P.cbmask);
+      }
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        if (warp * CW + 32 * b >= nt) break;  // the whole warp
+        const bool valid = w0 + 32 * b < nt;
+        const uint32_t cb = cbr[b];
+        uint32_t *mk = mask + (cb & (kLongHash - 1));
+        if (valid) atomicOr(mk, 1u << lane);
+        __syncwarp();
+        unsigned grp = valid ? *mk : 1u << lane;
+        const uint32_t base = mine[cb];
+        if (ncm > kLongHash) {  // drop the lanes of other c-mers
+          unsigned rem = grp & ~(1u << lane);
+          while (__any_sync(FULL, rem != 0)) {
+            const int j = rem ? __ffs(rem) - 1 : lane;
+            if (__shfl_sync(FULL, cb, j) != cb) grp &= ~(1u << j);
+            rem &= rem - 1;
+          }
+        }
+        __syncwarp();
+        if (valid) *mk = 0u;
+        if (valid && (grp & lt) == 0) mine[cb] = (uint16_t)(base + __popc(grp));
+        cbr[b] = cb | ((base + __popc(grp & lt)) << 16);
+        __syncwarp();
+      }
+      __syncthreads();
+      // exclusive scan over the warps of every bin, then over the bins
+      // (two bins per 32-bit word: no sum reaches 65536)
+      int carry = 0;
+      for (int i0 = 0; i0 < npair; i0 += kLongThreads) {
+        const int i = i0 + tid;
+        uint32_t run = 0;
+        if (i < npair) {
+          uint32_t c[kLongWarps];
+#pragma unroll
+          for (int w = 0; w < kLongWarps; ++w) c[w] = c32[w * npair + i];
+#pragma unroll
+          for (int w = 0; w < kLongWarps; ++w) {
+            c32[w * npair + i] = run;
+            run += c[w];
+          }
+        }
+        const int lo = (int)(run & 0xFFFFu), both = lo + (int)(run >> 16);
+        int inc = both;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(FULL, inc, o);
+          if (lane >= o) inc += y;
+        }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        int before = carry, all = 0;
+#pragma unroll
+        for (int w = 0; w < kLongWarps; ++w) {
+          const int c = wsum[w];
+          before += w < warp ? c : 0;
+          all += c;
+        }
+        if (i < npair) {
+          const int st = before + inc - both;
+          *reinterpret_cast<uint32_t *>(start + 2 * i) = (uint32_t)st | ((uint32_t)(st + lo) << 16);
+        }
+        carry += all;
+        __syncthreads();
+      }
+      if (tid == 0) start[ncm] = (uint16_t)carry;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const int w = warp * CW + b * 32 + lane;
+        if (w < nt) {
+          const uint32_t cb = cbr[b] & 0xFFFFu;
+          order[start[cb] + mine[cb] + (cbr[b] >> 16)] = (uint16_t)w;
+        }
+      }
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      // every complex bin's windows of this tile, in window order
+      for (int u = tid; u < P.nbin; u += kLongThreads) {
+        const int bin = u / P.m, idm = u - bin * P.m;
+        const int e0 = start[bin], e1 = start[bin + 1];
+        if (e0 == e1) continue;
+        const float2 *tb = tab + idm * TW;
+        float2 *h = reinterpret_cast<float2 *>(hist + hoff(u));
+        float2 a = *h;
+        int e = e0;
+        for (; e + 4 <= e1; e += 4) {
+          const float2 p0 = tb[order[e]], p1 = tb[order[e + 1]], p2 = tb[order[e + 2]], p3 = tb[order[e + 3]];
+          a = add2(add2(add2(add2(a, p0), p1), p2), p3);
+        }
+        for (; e < e1; ++e) a = add2(a, tb[order[e]]);
+        *h = a;
+      }
+      __syncthreads();
+    }
+    void *row = reinterpret_cast<unsigned char *>(dest) + rowbytes * it;
+    float *sc = scales ? scales + it : nullptr;
+    const bool fast = fast_rows(P);
+    if (warp == 0) {
+      float amax = 0.f;
+      finish_hist(P, hist, nrmv, norms + it * P.m, fast ? &amax : nullptr);
+      if (fast) {
+        if (lane == 0) *amax_s = amax;
+      } else {
+        write_row<OUT>(P, hist, nrmv, 0.f, row, sc, lane, 32);
+      }
+    }
+    __syncthreads();
+    if (fast) write_row<OUT>(P, hist, nrmv, *amax_s, row, sc, tid, kLongThreads);
+    __syncthreads();
+  }
+}
+
 // Bulk conversion, 16 values per thread and step.  VEC (both pointers 16-byte
 // aligned): 16-byte loads, all in flight before the first conversion, and one
 // 16-byte store, so a step moves 48 (fp16) or 80 (fp32) bytes per thread and
@@ -1142,7 +1405,7 @@ static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, in
     R2M_CUDA(cudaMallocAsync(&t, (size_t)P.m * P.nw * sizeof(float2), st));
     int nchunk = (P.nw + P.Wc - 1) / P.Wc;
     int tot = nchunk * P.m;
-    k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, t);
+    k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, P.nw, t);
     R2M_CUDA(cudaGetLastError());
     *gtable = t;
   }
@@ -1217,6 +1480,57 @@ static int launch_sparse_ref(const EncParams &P, void *dest, float *norms, float
   }
 }
 
+// Window tile of the block-per-fragment path for `items` fragments, 0 where
+// the one-warp path is the faster one (or the tile does not fit shared memory:
+// over 1,024 c-mers with m > 4).  A block's fragment takes about 4 us and 6 us
+// a tile with two blocks per SM; a warp takes about 1.3 us per 32 windows with
+// 20 resident per SM.  Measured (block against one-warp path, m = 1): 100
+// fragments of 700 bases 24 and 20 us, of 1,000 28 and 43, of 20,000 38 and
+// 506; 8,192 of 1,000 253 and 115, of 2,000 276 and 291, of 5,000 534 and
+// 1,226.  R2M_ENCODER=dense keeps the one-warp path.
+static int long_tile(const EncParams &P, int64_t items) {
+  const char *force = getenv("R2M_ENCODER");
+  if (force && strcmp(force, "dense") == 0) return 0;
+  if (P.nw <= 512) return 0;
+  int tile = P.m <= 2 && long_layout(P, 4096).total <= 220 * 1024 ? 4096 : 0;
+  if (tile == 0 && long_layout(P, 2048).total <= 220 * 1024) tile = 2048;
+  if (tile == 0) return 0;
+  const double sms = sm_count();
+  const double block_us = std::ceil(items / (2 * sms)) * (4.0 + 6.0 * ((P.nw + tile - 1) / tile));
+  const double warp_us = std::ceil(items / (20 * sms)) * 1.3 * ((P.nw + 31) / 32);
+  return block_us < warp_us ? tile : 0;
+}
+
+template <int OUT, int TW, bool REF>
+static int launch_long_as(const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin, int64_t batch,
+                          int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
+  auto kern = k_encode_long<OUT, TW, REF>;
+  const int smem = long_layout(P, TW).total;
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int per_sm = 1;
+  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLongThreads, smem));
+  const int64_t cap = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
+  const int pitch = (P.nw + 3) & ~1;  // rows start on 16 bytes, and the last pair of a row is whole
+  float2 *gt = nullptr;
+  R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&gt), (size_t)P.m * pitch * sizeof(float2), st));
+  const int tot = (P.nw + P.Wc - 1) / P.Wc * P.m;
+  k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, pitch, gt);
+  kern<<<(unsigned)(items < cap ? items : cap), kLongThreads, smem, st>>>(P, src, pos, nwin, batch, items, dest, norms,
+                                                                         scales, gt, pitch);
+  const cudaError_t e = cudaGetLastError();
+  cudaFreeAsync(gt, st);
+  if (e != cudaSuccess) return cuda_fail(e, "k_encode_long launch");
+  return R2M_OK;
+}
+
+template <int OUT, bool REF>
+static int launch_long(int tile, const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin,
+                       int64_t batch, int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
+  if (tile == 4096)
+    return launch_long_as<OUT, 4096, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
+  return launch_long_as<OUT, 2048, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
+}
+
 template <int OUT>
 static int launch_frags(EncParams P, void *dest, float *norms, float *scales, const uint32_t *dnas,
                         int64_t n, cudaStream_t st) {
@@ -1228,6 +1542,8 @@ static int launch_frags(EncParams P, void *dest, float *norms, float *scales, co
       default: return launch_sparse_frags<OUT, 8>(P, dest, norms, scales, dnas, n, st);
     }
   }
+  if (const int tile = long_tile(P, n))
+    return launch_long<OUT, false>(tile, P, dnas, nullptr, 0, 0, n, dest, norms, scales, st);
   int grid, block;
   size_t smem;
   float2 *gt = nullptr;
@@ -1251,6 +1567,8 @@ static int launch_ref(EncParams P, void *dest, float *norms, float *scales, cons
       default: return launch_sparse_ref<OUT, 8>(P, dest, norms, scales, genome, pos, nwin, batch, st);
     }
   }
+  if (const int tile = long_tile(P, 2 * nwin))
+    return launch_long<OUT, true>(tile, P, genome, pos, nwin, batch, 2 * nwin, dest, norms, scales, st);
   int grid, block;
   size_t smem;
   float2 *gt = nullptr;
@@ -1727,7 +2045,7 @@ extern "C" int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *can
   if (!P.table_in_smem) {
     R2M_CUDA(cudaMallocAsync(&gt, (size_t)P.m * P.nw * sizeof(float2), st));
     int nchunk = (P.nw + P.Wc - 1) / P.Wc;
-    k_phasor_table<<<(nchunk * P.m + 127) / 128, 128, 0, st>>>(P, gt);
+    k_phasor_table<<<(nchunk * P.m + 127) / 128, 128, 0, st>>>(P, P.nw, gt);
   }
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rescore_fp32, 128, smem);

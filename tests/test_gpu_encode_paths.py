@@ -1,6 +1,7 @@
-"""The encoder's dispatch: the register path of the FP32 rescoring and the bulk
-e4m3 conversion give the bytes of the general path they stand in for, at the
-edges of their tiles and on fragments whose windows crowd into few bins."""
+"""The encoder's dispatch: the block-per-fragment path for long fragments, the
+register path of the FP32 rescoring and the bulk e4m3 conversion give the bytes
+of the general path they stand in for, at the edges of their tiles and on
+fragments whose windows crowd into few bins."""
 import numpy as np
 import pytest
 import torch
@@ -11,6 +12,9 @@ import rotormap as rm
 from rotormap._lib import check, lib, ptr
 
 pytestmark = pytest.mark.gpu
+
+KINDS = {0: torch.float32, 1: torch.float16, 2: torch.uint8, 3: torch.uint8}
+
 
 def fragments(rng, n, k):
     """Random fragments, homopolymers and short tandem repeats, as codes."""
@@ -28,6 +32,52 @@ def pack(codes):
     full = np.zeros((n, (k + 15) // 16 * 16), np.uint32)
     full[:, :k] = codes
     return (full.reshape(n, -1, 16) << (2 * np.arange(16, dtype=np.uint32))).sum(2, dtype=np.uint32)
+
+
+def encode(words, k, s, m, c, kind, normalize):
+    n, rdim = words.shape[0], 2 * m * 4 ** c
+    out = torch.empty((n, rdim), dtype=KINDS[kind], device="cuda")
+    norms, scales = torch.empty((n, m), device="cuda"), torch.empty(n, device="cuda")
+    dw = torch.from_numpy(words.view(np.int32)).cuda()
+    check(lib().r2m_encode_frag_real_batch(ptr(out), kind, ptr(norms), ptr(scales), ptr(dw), n, k, s, m, c, normalize,
+                                           torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    got = [out.view(torch.uint8).cpu().numpy(), norms.cpu().numpy()]
+    return got + ([scales.cpu().numpy()] if kind == 3 else [])
+
+
+LONG = [(517, 5, 1, 5), (518, 5, 1, 5), (2055, 8, 4, 4), (2056, 8, 4, 4), (4100, 5, 1, 4), (4101, 5, 2, 3), (6149, 6, 3, 2),
+        (9001, 5, 1, 5), (2300, 8, 8, 3), (1500, 7, 1, 7), (700, 16, 1, 1)]
+
+
+@pytest.mark.parametrize("k,s,m,c", LONG)
+@pytest.mark.parametrize("kind,normalize", [(0, 0), (1, 0), (2, 0), (3, 0), (0, 1), (3, 2), (2, 3)])
+def test_long_fragments_equal_the_one_warp_path(k, s, m, c, kind, normalize, monkeypatch):
+    words = pack(fragments(np.random.default_rng(k + m), 9, k))
+    got = encode(words, k, s, m, c, kind, normalize)
+    monkeypatch.setenv("R2M_ENCODER", "dense")
+    for a, b in zip(got, encode(words, k, s, m, c, kind, normalize)):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("k,s,m,c,nwin,batch", [(1003, 5, 1, 5, 11, 4), (2500, 8, 4, 4, 3, 100), (4101, 5, 1, 4, 5, 1)])
+def test_long_index_windows_equal_the_one_warp_path(k, s, m, c, nwin, batch, monkeypatch):
+    rng = np.random.default_rng(k)
+    step = 61
+    genome = pack(fragments(rng, 6, k + step * nwin).reshape(1, -1))[0]
+    g = torch.from_numpy(np.concatenate([genome, np.zeros(4, np.uint32)]).view(np.int32)).cuda()
+    pos = torch.from_numpy(3 + step * np.arange(nwin, dtype=np.int64) * 5).cuda()
+    res = []
+    for path in ("auto", "dense"):
+        monkeypatch.setenv("R2M_ENCODER", path)
+        out = torch.empty((2 * nwin, 2 * m * 4 ** c), dtype=torch.uint8, device="cuda")
+        norms, scales = torch.empty((2 * nwin, m), device="cuda"), torch.empty(2 * nwin, device="cuda")
+        check(lib().r2m_encode_ref_windows(ptr(out), 3, ptr(norms), ptr(scales), ptr(g), ptr(pos), nwin, batch, k, s, m,
+                                           c, 0, torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        res.append([t.cpu().numpy() for t in (out, norms, scales)])
+    for a, b in zip(*res):
+        assert np.array_equal(a, b)
 
 
 @pytest.mark.parametrize("k,s,m,c", [(150, 8, 4, 4), (100, 8, 4, 3), (250, 8, 2, 4), (160, 5, 1, 5), (37, 5, 1, 4)])
