@@ -28,6 +28,7 @@
 #include <float.h>
 #include <limits.h>
 
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
@@ -44,7 +45,7 @@ constexpr int A_STAGE = BM * BK;  // 16 KiB
 constexpr int B_STAGE = BN * BK;  // 32 KiB
 constexpr int TMEM_COLS = 512;
 constexpr long long WAIT_LIMIT = 4000000000LL;  // clock cycles (~2 s)
-constexpr int MAX_LISTS = 128;  // partial lists per row (column splits x epilogue halves)
+constexpr int MAX_LISTS = 320;  // partial lists per row (column splits x epilogue halves)
 // Epilogue forms of both kernels: 4 * H epilogue warps.  With H = 2 two warps
 // share each TMEM lane quarter, each draining one half (128 columns) of
 // every tile into its own reservoir, so a (read tile, column split) unit
@@ -923,14 +924,15 @@ static void launch_merge_as(const GemmArgs &g, int lists, int KT, const float *s
 // Merge the `lists` partial lists a launch with arguments g left per row.
 static int launch_merge(const GemmArgs &g, int lists, int KT, const float *scaleA, float *vals, int *locs,
                         cudaStream_t st) {
-  static_assert(MAX_LISTS <= 32 * 4, "the widest merge holds 128 lists");
+  static_assert(MAX_LISTS <= 32 * 10, "the widest merge holds 320 lists");
   if (g.score_mode != R2M_SCORE_SCALED) scaleA = nullptr;
   if (lists <= 4) launch_merge_as<4, 1>(g, lists, KT, scaleA, vals, locs, st);
   else if (lists <= 8) launch_merge_as<8, 1>(g, lists, KT, scaleA, vals, locs, st);
   else if (lists <= 16) launch_merge_as<8, 2>(g, lists, KT, scaleA, vals, locs, st);
   else if (lists <= 32) launch_merge_as<32, 1>(g, lists, KT, scaleA, vals, locs, st);
   else if (lists <= 64) launch_merge_as<32, 2>(g, lists, KT, scaleA, vals, locs, st);
-  else launch_merge_as<32, 4>(g, lists, KT, scaleA, vals, locs, st);
+  else if (lists <= 128) launch_merge_as<32, 4>(g, lists, KT, scaleA, vals, locs, st);
+  else launch_merge_as<32, 10>(g, lists, KT, scaleA, vals, locs, st);
   R2M_CUDA(cudaGetLastError());
   return R2M_OK;
 }
@@ -988,17 +990,24 @@ static size_t gemm_smem_bytes(int H) {
          CAND_BYTES;
 }
 
-// Column splits for a given number of read tiles.  The single-CTA kernel,
-// or fewer read tiles than half the CTA pairs: enough units to keep every
-// CTA busy, chosen to minimise the last-wave imbalance.  The CTA-pair kernel
-// with more read tiles runs power-bound, where a wave with a few idle pairs
-// loses little (the busy ones clock higher) but every doubling of the splits
-// costs about 9% at equal wave use (measured against 3,297,890 columns,
-// 16,384-65,536 reads: one split beat the imbalance-minimising choice by 8-18%
-// below 65,536 reads); so there the splits maximise
-// units / (waves x pairs) x 0.91^log2(splits) over 1..8.
-static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max_splits = MAX_LISTS,
-                         bool pair = false) {
+// Column splits for a given number of read tiles.
+//
+// At least half as many read tiles as CTA pairs: the board is power-bound, a
+// last wave with a few idle pairs loses little (the busy ones clock higher)
+// but every doubling of the splits costs about 9% at equal wave use (20,000
+// reads x 300,007 columns, 79 tiles: 13.7 ms with one split, 9.8 with 5, 9.9
+// with 10), so the splits maximise units / (waves x pairs) x
+// 0.91^log2(splits) over 1..8.
+//
+// Fewer read tiles: whole waves of equal units decide.  A unit takes its
+// column tiles plus about `fixed` more for filling its reservoirs (8 tiles of
+// 6.5 us up to 20 entries, 50 at 64), so the splits minimise waves x (tiles +
+// fixed); 4% per doubling of the waves covers the index reads that pairs in
+// different splits do not share.  Against the rule before (at least four units per CTA, capped at 64
+// splits): 100 reads x 1,000,003 columns 489 -> 336 us (148 splits, one per
+// SM), 1,000 x 300,007 575 -> 498 (18), 1,000 x 30,000 196 -> 103 (18),
+// 4,096 x 20,000 333 -> 182 (4), 4,096 x 500,000 at k = 64 4.9 -> 3.6 ms (4).
+static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max_splits, bool pair, int KT) {
   if (forced > 0) {
     int s = forced;
     if (s > n_tiles) s = n_tiles;
@@ -1007,8 +1016,8 @@ static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max
   }
   int cap = n_tiles < max_splits ? n_tiles : max_splits;
   if (cap < 1) cap = 1;
+  int best = 1;
   if (pair && 2 * m_tiles >= ctas) {
-    int best = 1;
     double best_score = -1.0;
     for (int s = 1; s <= 8 && s <= cap; ++s) {
       const long long units = (long long)m_tiles * s;
@@ -1021,17 +1030,18 @@ static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max
     }
     return best;
   }
-  int smin = (4 * ctas + m_tiles - 1) / m_tiles;
-  if (smin < 1) smin = 1;
-  if (smin > cap) smin = cap;
-  int best = smin;
-  double best_eff = -1.0;
-  for (int s = smin; s <= cap && s <= 2 * smin; ++s) {
-    long long units = (long long)m_tiles * s;
-    long long waves = (units + ctas - 1) / ctas;
-    double eff = (double)units / (double)(waves * ctas);
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
+  const int fixed = KT <= 20 ? 8 : KT <= 32 ? 16 : 50;
+  double best_cost = 0.0, weight = 0.0;
+  int waves = 0;
+  for (int s = 1; s <= cap; ++s) {
+    const int w = (m_tiles * s + ctas - 1) / ctas;
+    if (w != waves) {
+      waves = w;
+      weight = w * (1.0 + 0.04 * std::log2((double)w));
+    }
+    const double cost = weight * ((n_tiles + s - 1) / s + fixed);
+    if (s == 1 || cost < best_cost) {
+      best_cost = cost;
       best = s;
     }
   }
@@ -1121,6 +1131,7 @@ static int preload_kernels() {
   R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 1>));
   R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 2>));
   R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 4>));
+  R2M_CUDA(cudaFuncGetAttributes(&fa, k_merge_splits<32, 10>));
   done[dev] = true;
   return R2M_OK;
 }
@@ -1181,6 +1192,19 @@ static int pace_window_for(const r2m_tuning *tune) {
   return r < 0 ? 0 : r == 0 ? PACE_WINDOW : r;
 }
 
+// One allocation: `lists` partial lists of KT values and columns, then the
+// pacing slots.
+static cudaError_t alloc_workspace(size_t lists, int KT, float **vals, int **cols, long long **pace) {
+  unsigned char *p = nullptr;
+  const size_t part = lists * KT * sizeof(float);  // a multiple of 4 KB: lists come in tiles of 128
+  const cudaError_t e = cudaMalloc(&p, 2 * part + kPaceSlots * sizeof(long long));
+  if (e != cudaSuccess) return e;
+  *vals = reinterpret_cast<float *>(p);
+  *cols = reinterpret_cast<int *>(p + part);
+  *pace = reinterpret_cast<long long *>(p + 2 * part);
+  return cudaSuccess;
+}
+
 // Split lists the workspace must hold for any batch height up to rows_cap.
 static size_t lists_needed(int rows_cap, int n_tiles, int ctas, int forced, int mode, int KT) {
   size_t lists = 0;
@@ -1193,7 +1217,7 @@ static size_t lists_needed(int rows_cap, int n_tiles, int ctas, int forced, int 
     // either kernel may leave two partial lists per row and split
     (void)kind;
     const int H = KT <= 32 ? 2 : 1;
-    size_t l = (size_t)choose_splits(mt, n_tiles, c, forced, MAX_LISTS / H, kind == 2) * H * mt * tile;
+    size_t l = (size_t)choose_splits(mt, n_tiles, c, forced, MAX_LISTS / H, kind == 2, KT) * H * mt * tile;
     if (l > lists) lists = l;
   }
   return lists;
@@ -1286,20 +1310,13 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
   // workspace: the largest (read tiles x splits) any batch height can ask for
   size_t lists = lists_needed(rows_cap, e->n_tiles, e->ctas, e->forced_splits, e->mode, e->KT);
   e->part_lists = lists;
-  cudaError_t ce = cudaMalloc(&e->part_vals, lists * e->KT * sizeof(float));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->part_cols, lists * e->KT * sizeof(int));
-  if (ce == cudaSuccess) ce = cudaMalloc(&e->pace, kPaceSlots * sizeof(long long));
-  if (ce != cudaSuccess) {
-    cudaFree(e->part_vals);
-    cudaFree(e->part_cols);
+  if (alloc_workspace(lists, e->KT, &e->part_vals, &e->part_cols, &e->pace) != cudaSuccess) {
     delete e;
     return fail(R2M_ENOMEM, "engine workspace allocation failed");
   }
   rc = device_error_word(&e->err);
   if (rc) {
     cudaFree(e->part_vals);
-    cudaFree(e->part_cols);
-    cudaFree(e->pace);
     delete e;
     return rc;
   }
@@ -1309,9 +1326,7 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
 
 extern "C" int r2m_engine_destroy(r2m_engine *eng) {
   if (!eng) return R2M_OK;
-  cudaFree(eng->part_vals);
-  cudaFree(eng->part_cols);
-  cudaFree(eng->pace);
+  cudaFree(eng->part_vals);  // the whole workspace
   if (eng->timing)
     for (int i = 0; i < 3; ++i) cudaEventDestroy(eng->ev[i]);
   delete eng;
@@ -1328,17 +1343,18 @@ extern "C" int r2m_engine_set_tuning(r2m_engine *eng, const r2m_tuning *tune) {
   if (lists * KT > eng->part_lists * eng->KT) {  // grow the split workspace
     float *pv = nullptr;
     int *pc = nullptr;
-    cudaError_t ce = cudaMalloc(&pv, lists * KT * sizeof(float));
-    if (ce == cudaSuccess) ce = cudaMalloc(&pc, lists * KT * sizeof(int));
+    long long *pace = nullptr;
+    if (alloc_workspace(lists, KT, &pv, &pc, &pace) != cudaSuccess)
+      return fail(R2M_ENOMEM, "engine workspace allocation failed");
+    const cudaError_t ce = cudaDeviceSynchronize();
     if (ce != cudaSuccess) {
       cudaFree(pv);
-      return fail(R2M_ENOMEM, "engine workspace allocation failed");
+      return cuda_fail(ce, "cudaDeviceSynchronize");
     }
-    R2M_CUDA(cudaDeviceSynchronize());
     cudaFree(eng->part_vals);
-    cudaFree(eng->part_cols);
     eng->part_vals = pv;
     eng->part_cols = pc;
+    eng->pace = pace;
     eng->part_lists = lists;
   } else {
     eng->part_lists = eng->part_lists * eng->KT / KT;  // the same bytes hold more, shorter lists
@@ -1414,7 +1430,11 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.N = eng->N;
   g.n_tiles = eng->n_tiles;
   const int hmax = eng->KT <= 32 ? 2 : 1;
-  g.splits = choose_splits(g.num_m_tiles, eng->n_tiles, ctas_eff, eng->forced_splits, MAX_LISTS / hmax, kind == 2);
+  // (a rebound index of fewer columns may prefer more splits than the
+  // workspace was sized for)
+  const size_t room = eng->part_lists / ((size_t)hmax * g.num_m_tiles * tile);
+  g.splits = choose_splits(g.num_m_tiles, eng->n_tiles, ctas_eff, eng->forced_splits,
+                           (int)std::min<size_t>(MAX_LISTS / hmax, room), kind == 2, eng->KT);
   const int halves =
       eng->epi == 1 ? 1 : eng->epi == 2 ? hmax : epi_halves_for(kind, eng->KT, eng->n_tiles, g.splits);
   const int lists_per_row = halves * g.splits;  // partial lists each row leaves
@@ -1594,7 +1614,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   const int ctas_eff = kind == 2 ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
   const int hmax = KT <= 32 ? 2 : 1;
   // the engine's automatic schedule, with the splits cut to the scratch
-  int splits = choose_splits(m_tiles, n_tiles, ctas_eff, 0, MAX_LISTS / hmax, kind == 2);
+  int splits = choose_splits(m_tiles, n_tiles, ctas_eff, 0, MAX_LISTS / hmax, kind == 2, KT);
   int halves = epi_halves_for(kind, KT, n_tiles, splits);
   while (splits > 1 && (size_t)halves * splits * mpad > max_lists) {
     --splits;
