@@ -82,6 +82,8 @@ struct GemmArgs {
   uint32_t *err;
   long long *pace;  // CTA-pair kernel: per-pair progress (null = no pacing)
   int pace_window;  // column tiles a pair may run ahead of the slowest one
+  uint32_t *pub;    // shared row bounds (null = none): key of list l, row r at [l * mpad + r]
+  int conc;         // column splits whose lists share a bound
 };
 
 __device__ __forceinline__ int split_lo(int s, int n_tiles, int splits) {
@@ -98,14 +100,15 @@ struct Reservoir {
   float v[KT];
   int c[KT];
   float thr;
+  float floor;  // a later column at or below it is not among the row's top k (shared bound)
 
-  __device__ __forceinline__ void reset() {
+  __device__ __forceinline__ void reset(float bound) {
 #pragma unroll
     for (int i = 0; i < KT; ++i) {
       v[i] = -INFINITY;
       c[i] = INT_MAX;
     }
-    thr = -INFINITY;
+    thr = floor = bound;
   }
   // Columns arrive in increasing order, so an equal value goes behind the
   // kept one.  x <= v[KT-1] (-inf, a candidate that has since been beaten)
@@ -125,11 +128,87 @@ struct Reservoir {
       c[0] = col;
     }
   }
-  // v[k-1] by selects (a run-time index would move the list to memory)
-  __device__ __forceinline__ void update_thr(int k) {
-    thr = v[0];
+  // v[n-1] by selects (a run-time index would move the list to memory)
+  __device__ __forceinline__ float best(int n) const {
+    float x = v[0];
 #pragma unroll
-    for (int i = 1; i < KT; ++i) thr = i < k ? v[i] : thr;
+    for (int i = 1; i < KT; ++i) x = i < n ? v[i] : x;
+    return x;
+  }
+  __device__ __forceinline__ void update_thr(int k) { thr = fmaxf(best(k), floor); }
+  __device__ __forceinline__ void raise_floor(float f) {
+    floor = fmaxf(floor, f);
+    thr = fmaxf(thr, f);
+  }
+};
+
+constexpr int BOUND_LISTS = 16;  // lists that share a bound at most (each reads them all)
+
+// Shared row bounds.  The lists that a row gathers at the same time (the
+// epilogue halves of the column splits in one wave) see a fraction of its
+// columns each, and their own k-th values say little: n columns in, a list of
+// S admits k (1 + ln(n / k)) candidates, S times what the row as a whole
+// needs.  So after every flush a list publishes its q-th best value, q =
+// ceil(k / S): S lists with q values each hold at least k values no smaller
+// than the least of the S published ones, so a column below that is out.  The
+// group's bound is read after tiles 1, 2, 3, 4, 6, 8, 12, ... of a unit, and
+// the bound of the wave before at the start of one.  Keys are ordered like the
+// values, 0 = nothing published; stale reads are only lower bounds, so no
+// ordering is needed, and results do not depend on what is seen when.  Measured
+// (whole search, own thresholds -> shared bounds): 1,000 reads x 300,007
+// columns 489 -> 472 us, 300 x 100,000 124 -> 113, 4,096 x 20,000 185 -> 164; at
+// k = 64 100 x 1,000,003 455 -> 411, 1,000 x 300,007 757 -> 654.
+__device__ __forceinline__ uint32_t bound_key(float x) {
+  const uint32_t u = __float_as_uint(x);
+  return (u >> 31) ? ~u : (u | 0x80000000u);
+}
+// The largest value below the one of `key`: candidates must exceed it.
+__device__ __forceinline__ float below_key(uint32_t key) {
+  const float x = __uint_as_float((key >> 31) ? key & 0x7FFFFFFFu : ~key);
+  if (x == 0.f) return __uint_as_float(0x80000001u);
+  return __uint_as_float(__float_as_uint(x) + (x > 0.f ? -1 : 1));
+}
+
+struct Bounds {
+  uint32_t *pub;             // GemmArgs::pub (null = none)
+  int group, mine, stride;   // elements of pub: the group's first key of this row, this list's key
+  int lists, q;
+
+  // Unit of column split sp, epilogue half `half` of H, row `row`.
+  __device__ __forceinline__ void init(const GemmArgs &g, int sp, int half, int H, int row) {
+    const int s0 = sp / g.conc * g.conc, s1 = min(s0 + g.conc, g.splits);
+    pub = row < g.nb ? g.pub : nullptr;
+    lists = (s1 - s0) * H;
+    q = (g.k + lists - 1) / lists;
+    stride = g.mpad;
+    group = s0 * H * stride + row;
+    mine = (sp * H + half) * stride + row;
+  }
+  // What a candidate must exceed by the n lists whose first key is at `at`.
+  __device__ __forceinline__ float bound(int at, int n) const {
+    if (pub == nullptr) return -INFINITY;
+    uint32_t m = 0xFFFFFFFFu;
+#pragma unroll 8
+    for (int l = 0; l < n; ++l) {
+      uint32_t x;
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(pub + at + l * stride) : "memory");
+      m = min(m, x);
+    }
+    return m == 0 ? -INFINITY : below_key(m);
+  }
+  __device__ __forceinline__ float group_bound() const { return lists > 1 ? bound(group, lists) : -INFINITY; }
+  // The bound of the group before (full: conc splits), or -inf for the first.
+  __device__ __forceinline__ float bound_before(int n) const {
+    return group >= n * stride ? bound(group - n * stride, n) : -INFINITY;
+  }
+  __device__ __forceinline__ void publish(float x) const {
+    if (pub != nullptr && x > -INFINITY)
+      asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(pub + mine), "r"(bound_key(x)) : "memory");
+  }
+  // Whether to read the group's bound after tile number `done` (1, 2, ...) of the unit.
+  static __device__ __forceinline__ bool due(int done) {
+    const int top = 31 - __clz(done);
+    return top <= 1 || (done & ((1 << (top - 1)) - 1)) == 0;
   }
 };
 
@@ -166,20 +245,33 @@ struct Candidates {
         : "f"(x), "f"(thr), "r"(__float_as_uint(x)), "r"(col), "n"(STRIDE)
         : "memory");
   }
+  // Entry at byte offset o, or a value that no list takes.
+  __device__ __forceinline__ void load(uint32_t o, float &x, int &col) const {
+    uint32_t xb = 0xFF800000u;
+    col = 0;
+    if (base + o < end) asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(xb), "=r"(col) : "r"(base + o) : "memory");
+    x = __uint_as_float(xb);
+  }
   // Called by the whole warp.
   template <int KT>
-  __device__ __forceinline__ void flush(Reservoir<KT> &R, int k) {
+  __device__ __forceinline__ void flush(Reservoir<KT> &R, const Bounds &S, int k) {
     const unsigned FULL = 0xFFFFFFFFu;
     const uint32_t most = __reduce_max_sync(FULL, end - base);
+    float x;
+    int col;
+    load(0, x, col);
 #pragma unroll 1
     for (uint32_t o = 0; o < most; o += STRIDE) {
-      uint32_t xb = 0xFF800000u, col = 0;  // -inf: no candidate
-      if (base + o < end)
-        asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(xb), "=r"(col) : "r"(base + o) : "memory");
-      R.insert(__uint_as_float(xb), (int)col);
+      float next_x;
+      int next_col;
+      load(o + STRIDE, next_x, next_col);  // in flight during the insertion
+      R.insert(x, col);
+      x = next_x;
+      col = next_col;
     }
     end = base;
     R.update_thr(k);
+    S.publish(R.best(S.q));
   }
 };
 
@@ -218,7 +310,7 @@ __device__ __forceinline__ void apply_scales(float (&v)[32], const float4 (&s)[8
 // maxima of its four groups of 8 columns against the row's threshold decide,
 // for the warp as a whole, which groups have candidates.
 template <int KT, int H>
-__device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, float (&v)[32], long long c0,
+__device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, float (&v)[32], long long c0,
                                             long long N, bool tail, bool f16, int k) {
   const unsigned FULL = 0xFFFFFFFFu;
   if (tail) {
@@ -241,7 +333,7 @@ __device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, 
     if (__any_sync(FULL, m[q] > R.thr)) {
 #pragma unroll
       for (int j = 8 * q; j < 8 * q + 8; ++j) Q.append(f16 ? round_f16(v[j]) : v[j], R.thr, (int)(c0 + j));
-      if (__any_sync(FULL, Q.end > Q.limit)) Q.flush(R, k);
+      if (__any_sync(FULL, Q.end > Q.limit)) Q.flush(R, S, k);
     }
   }
 }
@@ -252,7 +344,7 @@ __device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, 
 // scales of chunk i + 1 are in flight while chunk i is scored.  Every load is
 // waited for before returning, so the caller may release the accumulator.
 template <int KT, int H, int CH>
-__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
                                            const float *scaleB, bool scaled, bool f16, int k) {
   static_assert(CH % 2 == 0, "chunks are drained in pairs");
   const bool tail = c_first + 32LL * CH > N;
@@ -269,7 +361,7 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, u
     if (scaled) apply_scales(va, s);
     tmem_ld32(taddr + (uint32_t)(i + 1) * 32u, vb);
     if (scaled) load_scales(s, scaleB, c0 + 32, N, tail);
-    score_chunk(R, Q, va, c0, N, tail, f16, k);
+    score_chunk(R, Q, S, va, c0, N, tail, f16, k);
     __syncwarp();
     tmem_wait_ld_tied(vb);
     if (scaled) apply_scales(vb, s);
@@ -277,7 +369,7 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, u
       tmem_ld32(taddr + (uint32_t)(i + 2) * 32u, va);
       if (scaled) load_scales(s, scaleB, c0 + 64, N, tail);
     }
-    score_chunk(R, Q, vb, c0 + 32, N, tail, f16, k);
+    score_chunk(R, Q, S, vb, c0 + 32, N, tail, f16, k);
   }
 }
 
@@ -285,7 +377,7 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, u
 // budget has no room for a second chunk (two warps per scheduler cover the
 // TMEM latency), and for the 64-entry reservoir.
 template <int KT, int H, int CH>
-__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
                                                   const float *scaleB, bool scaled, bool f16, int k) {
   const bool tail = c_first + 32LL * CH > N;
 #pragma unroll 1
@@ -298,18 +390,18 @@ __device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H
     tmem_ld32(taddr + (uint32_t)i * 32u, v);
     tmem_wait_ld_tied(v);
     if (scaled) apply_scales(v, s);
-    score_chunk(R, Q, v, c0, N, tail, f16, k);
+    score_chunk(R, Q, S, v, c0, N, tail, f16, k);
   }
 }
 
 template <int KT, int H>
-__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, Candidates<H> &Q, uint32_t taddr, long long c_first, long long N,
+__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
                                       const float *scaleB, bool scaled, bool f16, int k) {
   constexpr int CH = BN / 32 / H;
   if constexpr (H == 1 && KT < 64)
-    drain_tile<KT, H, CH>(R, Q, taddr, c_first, N, scaleB, scaled, f16, k);
+    drain_tile<KT, H, CH>(R, Q, S, taddr, c_first, N, scaleB, scaled, f16, k);
   else
-    drain_tile_serial<KT, H, CH>(R, Q, taddr, c_first, N, scaleB, scaled, f16, k);
+    drain_tile_serial<KT, H, CH>(R, Q, S, taddr, c_first, N, scaleB, scaled, f16, k);
 }
 
 template <int KT, int H>
@@ -475,11 +567,13 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     bool ok = true;
     Reservoir<KT> R;
     Candidates<H> Q;
+    Bounds S;
     Q.init(cand, threadIdx.x - 64);
     for (int u = blockIdx.x; ok && u < num_units; u += gridDim.x) {
       const int mt = u % g.num_m_tiles, sp = u / g.num_m_tiles;
       const int t0 = split_lo(sp, g.n_tiles, g.splits), t1 = split_lo(sp + 1, g.n_tiles, g.splits);
-      R.reset();
+      S.init(g, sp, half, H, mt * BM + row_in_tile);
+      R.reset(u != (int)blockIdx.x ? S.bound_before(g.conc * H) : -INFINITY);
       for (int t = t0; t < t1; ++t) {
         bool w = mbar_wait_bounded(&acc_full[acc], acc_phase, abort_flag, WAIT_LIMIT);
         if (__any_sync(FULL, !w)) {
@@ -490,24 +584,26 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, Q, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
+        drain_acc<KT, H>(R, Q, S, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
+        if (t + 1 < t1 && S.due(t - t0 + 1)) R.raise_floor(S.group_bound());
       }
       if (!ok) break;
-      Q.flush(R, g.k);
+      Q.flush(R, S, g.k);
       const int row = mt * BM + row_in_tile;
       if (row < g.nb) {
         const size_t list = (size_t)sp * H + half;
         float *pv = g.part_vals + (list * g.mpad + row) * KT;
         int *pc = g.part_cols + (list * g.mpad + row) * KT;
+        // 16 bytes a store: a lane's list is contiguous, its neighbours' are not
 #pragma unroll
-        for (int j = 0; j < KT; ++j) {
-          pv[j] = R.v[j];
-          pc[j] = R.c[j];
+        for (int j = 0; j < KT; j += 4) {
+          *reinterpret_cast<float4 *>(pv + j) = make_float4(R.v[j], R.v[j + 1], R.v[j + 2], R.v[j + 3]);
+          *reinterpret_cast<int4 *>(pc + j) = make_int4(R.c[j], R.c[j + 1], R.c[j + 2], R.c[j + 3]);
         }
       }
     }
@@ -557,7 +653,7 @@ constexpr int STAGE2_BYTES = KCH * HALF_TILE;  // per operand and CTA
 // while the pairs stay within an L2's worth of tiles of each other.  Left
 // alone they drift apart over a long unit, and then every pair streams the
 // index from DRAM itself.  So each pair's producer publishes its position
-// (column tiles issued since the launch; -1 = not started, LLONG_MAX = done)
+// (1 + column tiles issued since the launch; 0 = not started, LLONG_MAX = done)
 // every PACE_EVERY tiles and, while it is more than `window` tiles ahead of
 // the slowest started pair, sleeps -- for at most PACE_CHECKS short naps.
 // Pacing only ever delays a pair a little: it never waits for a pair that is
@@ -575,13 +671,13 @@ constexpr int PACE_LOST = 8;     // windows behind which a pair is no longer wai
 
 __device__ __forceinline__ void pace_pair(long long *pace, int pair, int npairs, long long pos, int window) {
   volatile long long *p = pace;
-  p[pair] = pos;
+  p[pair] = ++pos;
   for (int it = 0; it < PACE_CHECKS; ++it) {
     const long long lost = pos - (long long)PACE_LOST * window;
     long long mn = LLONG_MAX;
     for (int q = 0; q < npairs; ++q) {
       const long long v = p[q];
-      if (v >= 0 && v >= lost && v < mn) mn = v;
+      if (v > 0 && v >= lost && v < mn) mn = v;
     }
     if (pos - mn <= window) return;
     __nanosleep(1000);
@@ -773,11 +869,13 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     bool ok = true;
     Reservoir<KT> R;
     Candidates<H> Q;
+    Bounds S;
     Q.init(cand, threadIdx.x - 64);
     for (int u = pair; ok && u < num_units; u += npairs) {
       const int mt = u % g.num_m_tiles, sp = u / g.num_m_tiles;
       const int t0 = split_lo(sp, g.n_tiles, g.splits), t1 = split_lo(sp + 1, g.n_tiles, g.splits);
-      R.reset();
+      S.init(g, sp, half, H, mt * 256 + (int)rank * 128 + row_in_tile);
+      R.reset(u != pair ? S.bound_before(g.conc * H) : -INFINITY);
       for (int t = t0; t < t1; ++t) {
         bool w = mbar_wait_bounded(&acc_full[acc], acc_phase, abort_flag, WAIT_LIMIT);
         if (__any_sync(FULL, !w)) {
@@ -788,24 +886,26 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
         }
         tc_fence_after();
         const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, Q, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
+        drain_acc<KT, H>(R, Q, S, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), 0));
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1u;
+        if (t + 1 < t1 && S.due(t - t0 + 1)) R.raise_floor(S.group_bound());
       }
       if (!ok) break;
-      Q.flush(R, g.k);
+      Q.flush(R, S, g.k);
       const int row = mt * 256 + (int)rank * 128 + row_in_tile;
       if (row < g.nb) {
         const size_t list = (size_t)sp * H + half;
         float *pv = g.part_vals + (list * g.mpad + row) * KT;
         int *pc = g.part_cols + (list * g.mpad + row) * KT;
+        // 16 bytes a store: a lane's list is contiguous, its neighbours' are not
 #pragma unroll
-        for (int j = 0; j < KT; ++j) {
-          pv[j] = R.v[j];
-          pc[j] = R.c[j];
+        for (int j = 0; j < KT; j += 4) {
+          *reinterpret_cast<float4 *>(pv + j) = make_float4(R.v[j], R.v[j + 1], R.v[j + 2], R.v[j + 3]);
+          *reinterpret_cast<int4 *>(pc + j) = make_int4(R.c[j], R.c[j + 1], R.c[j + 2], R.c[j + 3]);
         }
       }
     }
@@ -830,10 +930,15 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
 // number of lists, so that a row of a large batch (few lists) does not
 // occupy a whole warp: 65,536 rows of 4 lists 308 -> 44 us, 8,192 rows of 32
 // lists 39 -> 20, 16 to 200 rows of 128 lists 18 -> 12 (launch included).
+// It also puts the launch's row bounds and pacing slots back to zero for the
+// next launch.
 template <int G, int PER>
 __global__ void __launch_bounds__(256) k_merge_splits(const float *__restrict__ pv, const int *__restrict__ pc,
                                                      int lists, int mpad, int KT, int nb, int k,
-                                                     const float *__restrict__ scaleA, float *out_v, int *out_l) {
+                                                     const float *__restrict__ scaleA, float *out_v, int *out_l,
+                                                     uint32_t *pub, long long *pace, int npace) {
+  if (pace != nullptr && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < npace; i += 256) pace[i] = 0;
   const int gl = threadIdx.x % G;
   const int row = blockIdx.x * (256 / G) + threadIdx.x / G;
   if (row >= nb) return;  // whole groups
@@ -854,6 +959,8 @@ __global__ void __launch_bounds__(256) k_merge_splits(const float *__restrict__ 
     c[q][0] = b.x, c[q][1] = b.y, c[q][2] = b.z, c[q][3] = b.w;
     taken[q] = 0;
   }
+  if (pub != nullptr)
+    for (int s = gl; s < lists; s += G) pub[(size_t)s * mpad + row] = 0u;
   const float sa = scaleA ? scaleA[row] : 1.0f;
   for (int r = 0; r < k; ++r) {
     float bv = v[0][0];
@@ -915,24 +1022,24 @@ __global__ void __launch_bounds__(256) k_merge_splits(const float *__restrict__ 
 
 template <int G, int PER>
 static void launch_merge_as(const GemmArgs &g, int lists, int KT, const float *scaleA, float *vals, int *locs,
-                            cudaStream_t st) {
+                            int npace, cudaStream_t st) {
   constexpr int rows = 256 / G;
   k_merge_splits<G, PER><<<(g.nb + rows - 1) / rows, 256, 0, st>>>(g.part_vals, g.part_cols, lists, g.mpad, KT, g.nb,
-                                                                  g.k, scaleA, vals, locs);
+                                                                  g.k, scaleA, vals, locs, g.pub, g.pace, npace);
 }
 
 // Merge the `lists` partial lists a launch with arguments g left per row.
 static int launch_merge(const GemmArgs &g, int lists, int KT, const float *scaleA, float *vals, int *locs,
-                        cudaStream_t st) {
+                        int npace, cudaStream_t st) {
   static_assert(MAX_LISTS <= 32 * 10, "the widest merge holds 320 lists");
   if (g.score_mode != R2M_SCORE_SCALED) scaleA = nullptr;
-  if (lists <= 4) launch_merge_as<4, 1>(g, lists, KT, scaleA, vals, locs, st);
-  else if (lists <= 8) launch_merge_as<8, 1>(g, lists, KT, scaleA, vals, locs, st);
-  else if (lists <= 16) launch_merge_as<8, 2>(g, lists, KT, scaleA, vals, locs, st);
-  else if (lists <= 32) launch_merge_as<32, 1>(g, lists, KT, scaleA, vals, locs, st);
-  else if (lists <= 64) launch_merge_as<32, 2>(g, lists, KT, scaleA, vals, locs, st);
-  else if (lists <= 128) launch_merge_as<32, 4>(g, lists, KT, scaleA, vals, locs, st);
-  else launch_merge_as<32, 10>(g, lists, KT, scaleA, vals, locs, st);
+  if (lists <= 4) launch_merge_as<4, 1>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else if (lists <= 8) launch_merge_as<8, 1>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else if (lists <= 16) launch_merge_as<8, 2>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else if (lists <= 32) launch_merge_as<32, 1>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else if (lists <= 64) launch_merge_as<32, 2>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else if (lists <= 128) launch_merge_as<32, 4>(g, lists, KT, scaleA, vals, locs, npace, st);
+  else launch_merge_as<32, 10>(g, lists, KT, scaleA, vals, locs, npace, st);
   R2M_CUDA(cudaGetLastError());
   return R2M_OK;
 }
@@ -1192,16 +1299,36 @@ static int pace_window_for(const r2m_tuning *tune) {
   return r < 0 ? 0 : r == 0 ? PACE_WINDOW : r;
 }
 
-// One allocation: `lists` partial lists of KT values and columns, then the
-// pacing slots.
-static cudaError_t alloc_workspace(size_t lists, int KT, float **vals, int **cols, long long **pace) {
+// Column splits whose lists share a row bound: those that run at the same time.
+static int bound_splits(int ctas, int m_tiles, int splits, int halves) {
+  const int c = std::max(1, std::min(ctas / m_tiles, splits)), most = BOUND_LISTS / halves;
+  const int groups = (c + most - 1) / most;
+  return (c + groups - 1) / groups;  // groups of equal size
+}
+
+// One allocation: the pacing slots and the row bounds (zero between launches),
+// then `lists` partial lists of KT values and columns.  The lists come in
+// tiles of 128, which keeps every part 16-byte aligned.
+struct Workspace {
+  long long *pace;
+  uint32_t *pub;
+  float *vals;
+  int *cols;
+};
+static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   unsigned char *p = nullptr;
-  const size_t part = lists * KT * sizeof(float);  // a multiple of 4 KB: lists come in tiles of 128
-  const cudaError_t e = cudaMalloc(&p, 2 * part + kPaceSlots * sizeof(long long));
+  const size_t part = lists * KT * sizeof(float), zero = kPaceSlots * sizeof(long long) + lists * sizeof(uint32_t);
+  cudaError_t e = cudaMalloc(&p, zero + 2 * part);
   if (e != cudaSuccess) return e;
-  *vals = reinterpret_cast<float *>(p);
-  *cols = reinterpret_cast<int *>(p + part);
-  *pace = reinterpret_cast<long long *>(p + 2 * part);
+  e = cudaMemset(p, 0, zero);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    return e;
+  }
+  w->pace = reinterpret_cast<long long *>(p);
+  w->pub = reinterpret_cast<uint32_t *>(p + kPaceSlots * sizeof(long long));
+  w->vals = reinterpret_cast<float *>(p + zero);
+  w->cols = reinterpret_cast<int *>(p + zero + part);
   return cudaSuccess;
 }
 
@@ -1243,11 +1370,11 @@ struct r2m_engine {
   CUtensorMap mapB128;  // 128-row box for the CTA-pair kernel
   int mode;             // 0 auto, 1 single-CTA kernel, 2 CTA-pair kernel
   int epi;              // CTA-pair epilogue: 0 auto, 1 four warps, 2 eight warps
-  float *part_vals;
-  int *part_cols;
+  Workspace ws;
   size_t part_lists;  // capacity in lists (rows x splits)
+  size_t pub_lists;   // row bounds the workspace holds
+  bool dirty;         // a launch whose merge did not follow may have left bounds behind
   uint32_t *err;
-  long long *pace;    // per-pair progress of the CTA-pair kernel (kPaceSlots)
   int pace_window;    // 0 = no pacing
   bool timing;        // record events around the two kernels of each call
   cudaEvent_t ev[3];
@@ -1310,13 +1437,15 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
   // workspace: the largest (read tiles x splits) any batch height can ask for
   size_t lists = lists_needed(rows_cap, e->n_tiles, e->ctas, e->forced_splits, e->mode, e->KT);
   e->part_lists = lists;
-  if (alloc_workspace(lists, e->KT, &e->part_vals, &e->part_cols, &e->pace) != cudaSuccess) {
+  if (alloc_workspace(lists, e->KT, &e->ws) != cudaSuccess) {
     delete e;
     return fail(R2M_ENOMEM, "engine workspace allocation failed");
   }
+  e->pub_lists = lists;
+  e->dirty = false;
   rc = device_error_word(&e->err);
   if (rc) {
-    cudaFree(e->part_vals);
+    cudaFree(e->ws.pace);
     delete e;
     return rc;
   }
@@ -1326,7 +1455,7 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
 
 extern "C" int r2m_engine_destroy(r2m_engine *eng) {
   if (!eng) return R2M_OK;
-  cudaFree(eng->part_vals);  // the whole workspace
+  cudaFree(eng->ws.pace);  // the whole workspace
   if (eng->timing)
     for (int i = 0; i < 3; ++i) cudaEventDestroy(eng->ev[i]);
   delete eng;
@@ -1341,20 +1470,18 @@ extern "C" int r2m_engine_set_tuning(r2m_engine *eng, const r2m_tuning *tune) {
   const int KT = kt_for(eng->k, tune);
   size_t lists = lists_needed(eng->rows_cap, eng->n_tiles, ctas, forced, mode, KT);
   if (lists * KT > eng->part_lists * eng->KT) {  // grow the split workspace
-    float *pv = nullptr;
-    int *pc = nullptr;
-    long long *pace = nullptr;
-    if (alloc_workspace(lists, KT, &pv, &pc, &pace) != cudaSuccess)
+    Workspace w;
+    if (alloc_workspace(lists, KT, &w) != cudaSuccess)
       return fail(R2M_ENOMEM, "engine workspace allocation failed");
     const cudaError_t ce = cudaDeviceSynchronize();
     if (ce != cudaSuccess) {
-      cudaFree(pv);
+      cudaFree(w.pace);
       return cuda_fail(ce, "cudaDeviceSynchronize");
     }
-    cudaFree(eng->part_vals);
-    eng->part_vals = pv;
-    eng->part_cols = pc;
-    eng->pace = pace;
+    cudaFree(eng->ws.pace);
+    eng->ws = w;
+    eng->pub_lists = lists;
+    eng->dirty = false;
     eng->part_lists = lists;
   } else {
     eng->part_lists = eng->part_lists * eng->KT / KT;  // the same bytes hold more, shorter lists
@@ -1443,8 +1570,8 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.k = eng->k;
   g.mpad = g.num_m_tiles * tile;
   g.scaleB = eng->scaleB;
-  g.part_vals = eng->part_vals;
-  g.part_cols = eng->part_cols;
+  g.part_vals = eng->ws.vals;
+  g.part_cols = eng->ws.cols;
   g.err = eng->err;
   if ((size_t)lists_per_row * g.mpad > eng->part_lists) return fail(R2M_ESTATE, "engine workspace too small");
   long long units = (long long)g.num_m_tiles * g.splits;
@@ -1453,16 +1580,22 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.pace = nullptr;
   g.pace_window = 0;
   if (kind == 2 && eng->pace_window > 0 && ctas > 1 && ctas <= kPaceSlots) {
-    // every pair starts as "not started" (-1)
-    R2M_CUDA(cudaMemsetAsync(eng->pace, 0xFF, (size_t)ctas * sizeof(long long), st));
-    g.pace = eng->pace;
+    g.pace = eng->ws.pace;
     g.pace_window = eng->pace_window;
   }
+  g.pub = (size_t)lists_per_row * g.mpad <= eng->pub_lists ? eng->ws.pub : nullptr;
+  g.conc = bound_splits(ctas, g.num_m_tiles, g.splits, halves);
+  // bounds and pacing slots are zero here: the merge of the launch before left
+  // them so, unless it never ran
+  if (eng->dirty)
+    R2M_CUDA(cudaMemsetAsync(eng->ws.pace, 0, kPaceSlots * sizeof(long long) + eng->pub_lists * sizeof(uint32_t), st));
+  eng->dirty = true;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[0], st));
   rc = dispatch_gemm(kind, halves, eng->KT, mapA, eng->mapB, eng->mapB128, g, ctas, st);
   if (rc) return rc;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[1], st));
-  if ((rc = launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, st))) return rc;
+  if ((rc = launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, ctas, st))) return rc;
+  eng->dirty = false;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[2], st));
   return R2M_OK;
 }
@@ -1642,17 +1775,24 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   const int ctas = (int)(units < ctas_eff ? units : ctas_eff);
   g.pace = nullptr;
   g.pace_window = 0;
-  // the error word must start at zero; the partial lists are fully
-  // rewritten by the kernel before the merge reads them
+  // the error word, the pacing slots and the row bounds must start at zero;
+  // the partial lists are fully rewritten by the kernel before the merge
+  // reads them.  Bounds go behind the lists where they fit.
   R2M_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
   if (kind == 2 && ctas > 1 && ctas <= kPaceSlots) {
-    R2M_CUDA(cudaMemsetAsync(pace, 0xFF, (size_t)ctas * sizeof(long long), st));  // "not started"
+    R2M_CUDA(cudaMemsetAsync(pace, 0, (size_t)ctas * sizeof(long long), st));
     g.pace = pace;
     g.pace_window = PACE_WINDOW;
   }
+  g.pub = nullptr;
+  g.conc = bound_splits(ctas, m_tiles, splits, halves);
+  if (nlists * (list_bytes + sizeof(uint32_t)) <= kNoAllocScratchBytes - kNoAllocPaceBytes) {
+    g.pub = reinterpret_cast<uint32_t *>(lists + nlists * list_bytes);
+    R2M_CUDA(cudaMemsetAsync(g.pub, 0, nlists * sizeof(uint32_t), st));
+  }
   rc = dispatch_gemm(kind, halves, KT, mapA, mapB, mapB128, g, ctas, st);
   if (rc) return rc;
-  if ((rc = launch_merge(g, halves * splits, KT, d_scaleA, d_vals, d_locs, st))) return rc;
+  if ((rc = launch_merge(g, halves * splits, KT, d_scaleA, d_vals, d_locs, ctas, st))) return rc;
   k_noalloc_poison<<<64, 256, 0, st>>>(err, d_vals, d_locs, (long long)nb * k);
   R2M_CUDA(cudaGetLastError());
   return R2M_OK;
