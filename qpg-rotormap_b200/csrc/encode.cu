@@ -28,6 +28,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -1038,8 +1039,16 @@ __host__ __device__ inline size_t sparse_table_bytes(const EncParams &P) {
   return ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
 }
 
+// Warps per block, by the copies m.  Shared memory bounds the residency (a
+// warp's area is about 6 KB at m = 4, the phasor table 4.5 KB a block at 150
+// bases): at m = 4 two blocks of 18 warps per SM share two tables where four of
+// 8 warps held four, 36 warps instead of 32.  65,536 reads of 150 bases 119.1
+// -> 114.5 us, of 250 bases 206 -> 186; 1,000,000 index columns of 150 bases
+// 1,694 -> 1,613 us, 200,000 of 250 bases 614 -> 533.
+__host__ __device__ constexpr int sparse_warps(int m) { return m == 4 ? 18 : 8; }
+
 template <int OUT, int M>
-__global__ void __launch_bounds__(256) k_encode_sparse(EncParams P, const uint32_t *__restrict__ dnas, int64_t n,
+__global__ void __launch_bounds__(32 * sparse_warps(M), M == 4 ? 2 : M < 4 ? 4 : 1) k_encode_sparse(EncParams P, const uint32_t *__restrict__ dnas, int64_t n,
                                                        void *dest, float *norms, float *scales) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2 *table = reinterpret_cast<float2 *>(smem);
@@ -1061,7 +1070,7 @@ __global__ void __launch_bounds__(256) k_encode_sparse(EncParams P, const uint32
 }
 
 template <int OUT, int M>
-__global__ void __launch_bounds__(256, M <= 4 ? 4 : 1) k_encode_sparse_ref(EncParams P, const uint32_t *__restrict__ genome,
+__global__ void __launch_bounds__(32 * sparse_warps(M), M == 4 ? 2 : M < 4 ? 4 : 1) k_encode_sparse_ref(EncParams P, const uint32_t *__restrict__ genome,
                                                            const int64_t *__restrict__ win_pos, int64_t nwin,
                                                            int64_t batch, void *dest, float *norms,
                                                            float *scales) {
@@ -1089,10 +1098,13 @@ __global__ void __launch_bounds__(256, M <= 4 ? 4 : 1) k_encode_sparse_ref(EncPa
     const int64_t bt = i / batch, off = i - bt * batch;
     const int64_t nb = min(batch, nwin - bt * batch);
     const int64_t colf = 2 * bt * batch + off, colr = colf + nb;
-    sparse_fragment<OUT, M>(P, table, warea, fw, reinterpret_cast<unsigned char *>(dest) + rowbytes * colf,
-                            norms + colf * M, scales ? scales + colf : nullptr);
-    sparse_fragment<OUT, M>(P, table, warea, rcw, reinterpret_cast<unsigned char *>(dest) + rowbytes * colr,
-                            norms + colr * M, scales ? scales + colr : nullptr);
+    // one copy of the encoder's code for both strands (two cost 4%: fetching it)
+#pragma unroll 1
+    for (int strand = 0; strand < 2; ++strand) {
+      const int64_t col = strand ? colr : colf;
+      sparse_fragment<OUT, M>(P, table, warea, strand ? rcw : fw, reinterpret_cast<unsigned char *>(dest) + rowbytes * col,
+                              norms + col * M, scales ? scales + col : nullptr);
+    }
   }
 }
 
@@ -1434,8 +1446,15 @@ template <typename KernelFn>
 static int sparse_grid(KernelFn kern, const EncParams &P, int outb, int64_t nwork, int *grid, int *block,
                        size_t *smem) {
   const SparseLayout L = sparse_layout(P.c, P.m, P.sp_nslot, outb);
-  int wpb = 8;
-  while (wpb > 1 && sparse_table_bytes(P) + (size_t)L.warp * wpb > 200 * 1024) wpb >>= 1;
+  // as many warps as fit, at m = 4 in two blocks per SM unless one larger block
+  // holds more
+  const size_t tb = sparse_table_bytes(P), most = 200 * 1024, half = 113 * 1024;
+  auto fit = [&](size_t bytes) {
+    return bytes > tb ? (int)std::min<size_t>(sparse_warps(P.m), (bytes - tb) / L.warp) : 0;
+  };
+  int wpb = fit(most);
+  if (P.m == 4 && 2 * fit(half) >= wpb) wpb = fit(half);
+  if (wpb < 1) wpb = 1;
   *block = 32 * wpb;
   *smem = sparse_table_bytes(P) + (size_t)L.warp * wpb;
   R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
