@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const
 // Bulk conversion, 16 values per thread and step.  VEC (both pointers 16-byte
 // aligned): 16-byte loads, all in flight before the first conversion, and one
 // 16-byte store, so a step moves 48 (fp16) or 80 (fp32) bytes per thread and
-// the pass is bound by HBM: 8,192 x 2,048 fp16 values in 12.3 us (4.1 TB/s,
+// the pass is bound by HBM: 8,192 x 2,048 fp16 values in 10.9 us (4.6 TB/s,
 // launch included), against 63.5 us with one value per load and one byte per
 // store.  Other alignments and the tail take one value at a time, consecutive
 // lanes on consecutive values.
@@ -1399,6 +1399,7 @@ template <typename S, bool VEC>
 __global__ void __launch_bounds__(256) k_to_e4m3(uint8_t *__restrict__ dst, const S *__restrict__ src, int64_t count) {
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
   const int64_t nvec = VEC ? count >> 4 : 0;
+#pragma unroll 2
   for (int64_t i = t0; i < nvec; i += nt) {
     constexpr int NQ = sizeof(S);  // 16-byte loads per 16 values
     union {
@@ -1639,7 +1640,9 @@ static int launch_ref(EncParams P, void *dest, float *norms, float *scales, cons
 template <typename S>
 static int launch_to_e4m3(uint8_t *dst, const S *src, int64_t count, cudaStream_t st) {
   const bool vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0;
-  const int64_t per_block = vec ? 4096 : 256;
+  // fp16: two steps a thread, both in flight (12.2 -> 10.9 us for 8,192 x 2,048
+  // values, 65.7 -> 61.2 for 65,536 x 2,048; no gain for fp32's wider steps)
+  const int64_t per_block = vec ? (sizeof(S) == 2 && count >= (1 << 22) ? 8192 : 4096) : 256;
   int64_t blocks = (count + per_block - 1) / per_block;
   if (blocks > (1 << 20)) blocks = 1 << 20;
   if (vec) k_to_e4m3<S, true><<<(unsigned)blocks, 256, 0, st>>>(dst, src, count);
