@@ -1127,8 +1127,9 @@ static size_t gemm_smem_bytes(int H) {
 // Fewer read tiles: whole waves of equal units decide.  A unit takes its
 // column tiles plus about `fixed` more for filling its reservoirs (8 tiles of
 // 6.5 us up to 20 entries, 50 at 64), so the splits minimise waves x (tiles +
-// fixed); 4% per doubling of the waves covers the index reads that pairs in
-// different splits do not share.  Against the rule before (at least four units per CTA, capped at 64
+// fixed); 6% per doubling of the waves covers the index reads that pairs in
+// different splits do not share (8,192 x 619,001: 7.2 ms with 2 splits in one
+// wave, 7.6 with 9 in four).  Against the rule before (at least four units per CTA, capped at 64
 // splits): 100 reads x 1,000,003 columns 489 -> 336 us (148 splits, one per
 // SM), 1,000 x 300,007 575 -> 498 (18), 1,000 x 30,000 196 -> 103 (18),
 // 4,096 x 20,000 333 -> 182 (4), 4,096 x 500,000 at k = 64 4.9 -> 3.6 ms (4).
@@ -1162,7 +1163,7 @@ static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max
     const int w = (m_tiles * s + ctas - 1) / ctas;
     if (w != waves) {
       waves = w;
-      weight = w * (1.0 + 0.04 * std::log2((double)w));
+      weight = w * (1.0 + 0.06 * std::log2((double)w));
     }
     const double cost = weight * ((n_tiles + s - 1) / s + fixed);
     if (s == 1 || cost < best_cost) {
