@@ -38,7 +38,7 @@
 namespace r2m {
 
 constexpr int BM = 128;           // read rows per tile (TMEM lanes)
-constexpr int BN = 256;           // index columns per tile (TMEM fp32 columns)
+constexpr int BN = 256;           // index columns per tile at most (TMEM fp32 columns; GemmArgs::bn)
 constexpr int BK = 128;           // K bytes per stage (one 128-byte swizzle row)
 constexpr int STAGES = 4;
 constexpr int A_STAGE = BM * BK;  // 16 KiB
@@ -70,6 +70,7 @@ struct GemmArgs {
   int nb;
   int num_m_tiles;
   long long N;
+  int bn;  // columns per tile: 64, 128, 192 or 256
   int n_tiles;
   int splits;
   int num_kb;
@@ -356,23 +357,22 @@ __device__ __forceinline__ void score_chunk(Reservoir<KT> &R, Candidates<H> &Q, 
   }
 }
 
-// Drain this warp's CH chunks of one accumulator tile (TMEM address `taddr`
-// = its lane quarter and first chunk; columns c_first .. c_first + 32 CH - 1)
+// Drain this warp's `ch` chunks (an even number) of one accumulator tile (TMEM address `taddr`
+// = its lane quarter and first chunk; columns c_first .. c_first + 32 ch - 1)
 // into the row's reservoir.  Software-pipelined: the TMEM load and the column
 // scales of chunk i + 1 are in flight while chunk i is scored.  Every load is
 // waited for before returning, so the caller may release the accumulator.
-template <int KT, int H, int CH>
-__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
+template <int KT, int H>
+__device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, int ch, long long c_first, long long N,
                                            const float *scaleB, bool scaled, bool f16, int k) {
-  static_assert(CH % 2 == 0, "chunks are drained in pairs");
-  const bool tail = c_first + 32LL * CH > N;
+  const bool tail = c_first + 32LL * ch > N;
   float va[32], vb[32];
   float4 s[8];
   __syncwarp();
   tmem_ld32(taddr, va);
   if (scaled) load_scales(s, scaleB, c_first, N, tail);
 #pragma unroll 1
-  for (int i = 0; i < CH; i += 2) {
+  for (int i = 0; i < ch; i += 2) {
     const long long c0 = c_first + 32LL * i;
     __syncwarp();
     tmem_wait_ld_tied(va);
@@ -383,7 +383,7 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, c
     __syncwarp();
     tmem_wait_ld_tied(vb);
     if (scaled) apply_scales(vb, s);
-    if (i + 2 < CH) {
+    if (i + 2 < ch) {
       tmem_ld32(taddr + (uint32_t)(i + 2) * 32u, va);
       if (scaled) load_scales(s, scaleB, c0 + 64, N, tail);
     }
@@ -394,12 +394,12 @@ __device__ __forceinline__ void drain_tile(Reservoir<KT> &R, Candidates<H> &Q, c
 // The same, one chunk at a time: for the 8-warp form, whose 168-register
 // budget has no room for a second chunk (two warps per scheduler cover the
 // TMEM latency), and for the 64-entry reservoir.
-template <int KT, int H, int CH>
-__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
+template <int KT, int H>
+__device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, int ch, long long c_first, long long N,
                                                   const float *scaleB, bool scaled, bool f16, int k) {
-  const bool tail = c_first + 32LL * CH > N;
+  const bool tail = c_first + 32LL * ch > N;
 #pragma unroll 1
-  for (int i = 0; i < CH; ++i) {
+  for (int i = 0; i < ch; ++i) {
     const long long c0 = c_first + 32LL * i;
     float v[32];
     float4 s[8];
@@ -413,16 +413,15 @@ __device__ __forceinline__ void drain_tile_serial(Reservoir<KT> &R, Candidates<H
 }
 
 template <int KT, int H>
-__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, long long c_first, long long N,
+__device__ __forceinline__ void drain_acc(Reservoir<KT> &R, Candidates<H> &Q, const Bounds &S, uint32_t taddr, int ch, long long c_first, long long N,
                                       const float *scaleB, bool scaled, bool f16, int k) {
-  constexpr int CH = BN / 32 / H;
   if constexpr (H == 1 && KT < 64)
-    drain_tile<KT, H, CH>(R, Q, S, taddr, c_first, N, scaleB, scaled, f16, k);
+    drain_tile<KT, H>(R, Q, S, taddr, ch, c_first, N, scaleB, scaled, f16, k);
   else
-    drain_tile_serial<KT, H, CH>(R, Q, S, taddr, c_first, N, scaleB, scaled, f16, k);
+    drain_tile_serial<KT, H>(R, Q, S, taddr, ch, c_first, N, scaleB, scaled, f16, k);
 }
 
-template <int KT, int H>
+template <int KT, int H, bool NARROW>
 __global__ void __launch_bounds__(epi_threads(H), 1)
     k_gemm_topk(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 GemmArgs g) {
@@ -470,6 +469,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   const uint32_t tmem_base = *tmem_slot;
 
   const int num_units = g.num_m_tiles * g.splits;
+  const int bn = NARROW ? g.bn : BN;  // columns per tile
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
@@ -489,9 +489,9 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&full[stage], A_STAGE + B_STAGE);
+            mbar_arrive_expect_tx(&full[stage], A_STAGE + (uint32_t)(bn * BK));
             tma_load_2d(sA + stage * A_STAGE, &tmA, &full[stage], kb * BK, mt * BM);
-            tma_load_2d(sB + stage * B_STAGE, &tmB, &full[stage], kb * BK, t * BN);
+            tma_load_2d(sB + stage * B_STAGE, &tmB, &full[stage], kb * BK, t * bn);
             ++issued;
             if (++stage == STAGES) {
               stage = 0;
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t idesc = idesc_e4m3_f32(BM, BN);
+      const uint32_t idesc = idesc_e4m3_f32(BM, bn);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -574,9 +574,9 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     __syncwarp();
   } else {
     // ------------------------------------------------ epilogue (top-k)
-    constexpr int CH = BN / 32 / H;  // 32-column chunks per warp and tile
+    const int ch = bn / 32 / H;    // 32-column chunks per warp and tile
     const int quarter = warp & 3;    // TMEM lanes [32*quarter, 32*quarter+32)
-    const int half = (warp - 2) >> 2;  // tile chunks [CH half, CH half + CH)
+    const int half = (warp - 2) >> 2;  // tile chunks [ch half, ch half + ch)
     const int row_in_tile = quarter * 32 + lane;
     const bool f16 = g.score_mode == R2M_SCORE_F16;
     const bool scaled = g.score_mode == R2M_SCORE_SCALED;
@@ -601,8 +601,8 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
           break;
         }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, Q, S, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * ch * 32);
+        drain_acc<KT, H>(R, Q, S, taddr, ch, (long long)t * bn + half * ch * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[acc]);
@@ -703,7 +703,7 @@ __device__ __forceinline__ void pace_pair(long long *pace, int pair, int npairs,
 }
 // CTA-pair kernel: TMA warp, MMA warp and 4 * H epilogue warps (epilogue
 // forms above).
-template <int KT, int H>
+template <int KT, int H, bool NARROW>
 __global__ void __launch_bounds__(epi_threads(H), 1)
     k_gemm_topk2(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -753,6 +753,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int num_units = g.num_m_tiles * g.splits;
+  const int bn = NARROW ? g.bn : BN;  // columns per tile
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
@@ -777,12 +778,12 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
             }
             const uint32_t fbar = mapa_shared(smem_u32(&full[stage]), 0);
             const int nch = g.num_kb - kb < KCH ? g.num_kb - kb : KCH;
-            if (leader) mbar_arrive_expect_tx(&full[stage], 4 * HALF_TILE * nch);
+            if (leader) mbar_arrive_expect_tx(&full[stage], (uint32_t)(2 * HALF_TILE + bn * BK) * nch);
             for (int c = 0; c < nch; ++c) {
               tma_load_2d_pair(sA + stage * STAGE2_BYTES + c * HALF_TILE, &tmA, fbar, (kb + c) * BK,
                                mt * 256 + (int)rank * 128);
               tma_load_2d_pair(sB + stage * STAGE2_BYTES + c * HALF_TILE, &tmB, fbar, (kb + c) * BK,
-                               t * BN + (int)rank * 128);
+                               t * bn + (int)rank * (bn >> 1));
             }
             ++issued;
             if (++stage == STAGES2) {
@@ -813,7 +814,7 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer (leader CTA)
     if (lane == 0 && leader) {
-      const uint32_t idesc = idesc_e4m3_f32(256, BN);
+      const uint32_t idesc = idesc_e4m3_f32(256, bn);
       // descriptors of stage 0; a stage / chunk / K step offset adds its
       // 16-byte units to the start-address field
       const uint64_t dA0 = smem_desc_sw128(smem_u32(sA)), dB0 = smem_desc_sw128(smem_u32(sB));
@@ -876,9 +877,9 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
     __syncwarp();
   } else {
     // ------------------------------------------------ epilogue (both CTAs)
-    constexpr int CH = BN / 32 / H;        // 32-column chunks per warp and tile
+    const int ch = bn / 32 / H;          // 32-column chunks per warp and tile
     const int quarter = warp & 3;          // TMEM lanes this warp may read
-    const int half = (warp - 2) >> 2;      // tile chunks [CH half, CH half + CH)
+    const int half = (warp - 2) >> 2;      // tile chunks [ch half, ch half + ch)
     const int row_in_tile = quarter * 32 + lane;
     const bool f16 = g.score_mode == R2M_SCORE_F16;
     const bool scaled = g.score_mode == R2M_SCORE_SCALED;
@@ -903,8 +904,8 @@ __global__ void __launch_bounds__(epi_threads(H), 1)
           break;
         }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * CH * 32);
-        drain_acc<KT, H>(R, Q, S, taddr, (long long)t * BN + half * CH * 32, g.N, g.scaleB, scaled, f16, g.k);
+        const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * BN + half * ch * 32);
+        drain_acc<KT, H>(R, Q, S, taddr, ch, (long long)t * bn + half * ch * 32, g.N, g.scaleB, scaled, f16, g.k);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&acc_empty[acc]), 0));
@@ -1174,13 +1175,43 @@ static int choose_splits(int m_tiles, int n_tiles, int ctas, int forced, int max
   return best;
 }
 
-template <int KT, int H>
+// Tiles and splits of a launch over N columns.  When every unit is one or two
+// tiles, narrower tiles spread the columns over more SMs: a tile takes its
+// columns plus the reads loaded with it again (32 + 3/4 of them, measured in
+// columns) in loads and, per column, in first insertions.  256 -> 64 columns: 1
+// read x 2,000 31.4 -> 23.1 us, 16 x 5,000 33.3 -> 29.3, 129 x 2,000 42.0 ->
+// 28.6; 256 -> 192: 16 x 20,000 41.5 -> 39.4, 1,000 x 5,000 45.6 -> 43.5.
+struct ColumnPlan {
+  int bn, n_tiles, splits;
+};
+static ColumnPlan plan_columns(long long N, int nb, int m_tiles, int ctas, int forced, int max_splits, bool pair,
+                               int KT, bool narrow = true) {
+  ColumnPlan p;
+  p.bn = BN;
+  p.n_tiles = (int)((N + BN - 1) / BN);
+  p.splits = choose_splits(m_tiles, p.n_tiles, ctas, forced, max_splits, pair, KT);
+  const int per_unit = (p.n_tiles + p.splits - 1) / p.splits;
+  if (!narrow || forced > 0 || m_tiles * p.splits > ctas || per_unit > 2) return p;
+  const int most = std::max(1, std::min(ctas / m_tiles, max_splits)), again = 32 + 3 * std::min(nb, BM) / 4;
+  int best = per_unit * (BN + again);
+  for (int bn = 192; bn >= 64; bn -= 64) {
+    const int tiles = (int)((N + bn - 1) / bn), tau = (tiles + most - 1) / most;
+    if (tau * (bn + again) >= best) continue;
+    best = tau * (bn + again);
+    p.bn = bn;
+    p.n_tiles = tiles;
+    p.splits = (tiles + tau - 1) / tau;
+  }
+  return p;
+}
+
+template <int KT, int H, bool NARROW = false>
 static int launch_gemm(const CUtensorMap &mA, const CUtensorMap &mB, const GemmArgs &g, int ctas,
                        cudaStream_t st) {
   size_t smem = gemm_smem_bytes(H);
   // a function attribute is per device: set it on every launch (cheap)
-  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk<KT, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_gemm_topk<KT, H><<<ctas, epi_threads(H), smem, st>>>(mA, mB, g);
+  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk<KT, H, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_gemm_topk<KT, H, NARROW><<<ctas, epi_threads(H), smem, st>>>(mA, mB, g);
   R2M_CUDA(cudaGetLastError());
   return R2M_OK;
 }
@@ -1199,11 +1230,11 @@ static int epi_halves_for(int kind, int KT, int n_tiles, int splits) {
   return (n_tiles + splits - 1) / splits <= SHORT_UNIT_TILES ? 2 : 1;
 }
 
-template <int KT, int H>
+template <int KT, int H, bool NARROW = false>
 static int launch_gemm2(const CUtensorMap &mA, const CUtensorMap &mB, const GemmArgs &g, int pairs,
                         cudaStream_t st) {
   size_t smem = gemm2_smem_bytes(H);
-  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk2<KT, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk2<KT, H, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(epi_threads(H), 1, 1);
@@ -1216,7 +1247,7 @@ static int launch_gemm2(const CUtensorMap &mA, const CUtensorMap &mB, const Gemm
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  R2M_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_topk2<KT, H>, mA, mB, g));
+  R2M_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_topk2<KT, H, NARROW>, mA, mB, g));
   return R2M_OK;
 }
 
@@ -1238,16 +1269,20 @@ static int preload_kernels() {
   R2M_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(mu);
   if (dev < 0 || dev >= 64 || done[dev]) return R2M_OK;
-#define R2M_PRELOAD1(KT, H)                                                                    \
-  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk<KT, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+#define R2M_PRELOAD1(KT, H, NARROW)                                                                    \
+  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk<KT, H, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 (int)gemm_smem_bytes(H)))
-#define R2M_PRELOAD2(KT, H)                                                                     \
-  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk2<KT, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+#define R2M_PRELOAD2(KT, H, NARROW)                                                                     \
+  R2M_CUDA(cudaFuncSetAttribute(k_gemm_topk2<KT, H, NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 (int)gemm2_smem_bytes(H)))
-  R2M_PRELOAD1(8, 1); R2M_PRELOAD1(16, 1); R2M_PRELOAD1(20, 1); R2M_PRELOAD1(32, 1); R2M_PRELOAD1(64, 1);
-  R2M_PRELOAD1(8, 2); R2M_PRELOAD1(16, 2); R2M_PRELOAD1(20, 2); R2M_PRELOAD1(32, 2);
-  R2M_PRELOAD2(8, 1); R2M_PRELOAD2(16, 1); R2M_PRELOAD2(20, 1); R2M_PRELOAD2(32, 1); R2M_PRELOAD2(64, 1);
-  R2M_PRELOAD2(8, 2); R2M_PRELOAD2(16, 2); R2M_PRELOAD2(20, 2); R2M_PRELOAD2(32, 2);
+#define R2M_PRELOAD(KT, H, NARROW) \
+  R2M_PRELOAD1(KT, H, NARROW);     \
+  R2M_PRELOAD2(KT, H, NARROW)
+  R2M_PRELOAD(8, 1, false); R2M_PRELOAD(16, 1, false); R2M_PRELOAD(20, 1, false); R2M_PRELOAD(32, 1, false);
+  R2M_PRELOAD(8, 2, false); R2M_PRELOAD(16, 2, false); R2M_PRELOAD(20, 2, false); R2M_PRELOAD(32, 2, false);
+  R2M_PRELOAD(8, 2, true); R2M_PRELOAD(16, 2, true); R2M_PRELOAD(20, 2, true); R2M_PRELOAD(32, 2, true);
+  R2M_PRELOAD(64, 1, false); R2M_PRELOAD(64, 1, true);
+#undef R2M_PRELOAD
 #undef R2M_PRELOAD1
 #undef R2M_PRELOAD2
   cudaFuncAttributes fa;
@@ -1271,40 +1306,41 @@ static int kernel_kind(int mode, int nb) {
 }
 
 // Launch the fused kernel of `kind` (1 single-CTA, 2 CTA pairs) with
-// `halves` epilogue halves for the reservoir size KT.
+// `halves` epilogue halves for the reservoir size KT.  Tiles narrower than BN
+// have instances of their own (a run-time tile width costs the others 1%), for
+// the most halves of a reservoir size.
+template <int KT, int H, bool NARROW = false>
+static int launch_kind(int kind, const CUtensorMap &mA, const CUtensorMap &mB, const CUtensorMap &mB128,
+                       const GemmArgs &g, int ctas, cudaStream_t st) {
+  return kind == 2 ? launch_gemm2<KT, H, NARROW>(mA, mB128, g, ctas, st)
+                   : launch_gemm<KT, H, NARROW>(mA, mB, g, ctas, st);
+}
 static int dispatch_gemm(int kind, int halves, int KT, const CUtensorMap &mA, const CUtensorMap &mB,
                          const CUtensorMap &mB128, const GemmArgs &g, int ctas, cudaStream_t st) {
-  if (kind == 2) {
-    if (halves == 2) {
-      switch (KT) {
-        case 8: return launch_gemm2<8, 2>(mA, mB128, g, ctas, st);
-        case 16: return launch_gemm2<16, 2>(mA, mB128, g, ctas, st);
-        case 20: return launch_gemm2<20, 2>(mA, mB128, g, ctas, st);
-        default: return launch_gemm2<32, 2>(mA, mB128, g, ctas, st);
-      }
-    }
+  if (g.bn != BN) {
+    if (halves != (KT <= 32 ? 2 : 1)) return fail(R2M_ESTATE, "narrow tiles need the widest epilogue");
     switch (KT) {
-      case 8: return launch_gemm2<8, 1>(mA, mB128, g, ctas, st);
-      case 16: return launch_gemm2<16, 1>(mA, mB128, g, ctas, st);
-      case 20: return launch_gemm2<20, 1>(mA, mB128, g, ctas, st);
-      case 32: return launch_gemm2<32, 1>(mA, mB128, g, ctas, st);
-      default: return launch_gemm2<64, 1>(mA, mB128, g, ctas, st);
+      case 8: return launch_kind<8, 2, true>(kind, mA, mB, mB128, g, ctas, st);
+      case 16: return launch_kind<16, 2, true>(kind, mA, mB, mB128, g, ctas, st);
+      case 20: return launch_kind<20, 2, true>(kind, mA, mB, mB128, g, ctas, st);
+      case 32: return launch_kind<32, 2, true>(kind, mA, mB, mB128, g, ctas, st);
+      default: return launch_kind<64, 1, true>(kind, mA, mB, mB128, g, ctas, st);
     }
   }
   if (halves == 2) {
     switch (KT) {
-      case 8: return launch_gemm<8, 2>(mA, mB, g, ctas, st);
-      case 16: return launch_gemm<16, 2>(mA, mB, g, ctas, st);
-      case 20: return launch_gemm<20, 2>(mA, mB, g, ctas, st);
-      default: return launch_gemm<32, 2>(mA, mB, g, ctas, st);
+      case 8: return launch_kind<8, 2>(kind, mA, mB, mB128, g, ctas, st);
+      case 16: return launch_kind<16, 2>(kind, mA, mB, mB128, g, ctas, st);
+      case 20: return launch_kind<20, 2>(kind, mA, mB, mB128, g, ctas, st);
+      default: return launch_kind<32, 2>(kind, mA, mB, mB128, g, ctas, st);
     }
   }
   switch (KT) {
-    case 8: return launch_gemm<8, 1>(mA, mB, g, ctas, st);
-    case 16: return launch_gemm<16, 1>(mA, mB, g, ctas, st);
-    case 20: return launch_gemm<20, 1>(mA, mB, g, ctas, st);
-    case 32: return launch_gemm<32, 1>(mA, mB, g, ctas, st);
-    default: return launch_gemm<64, 1>(mA, mB, g, ctas, st);
+    case 8: return launch_kind<8, 1>(kind, mA, mB, mB128, g, ctas, st);
+    case 16: return launch_kind<16, 1>(kind, mA, mB, mB128, g, ctas, st);
+    case 20: return launch_kind<20, 1>(kind, mA, mB, mB128, g, ctas, st);
+    case 32: return launch_kind<32, 1>(kind, mA, mB, mB128, g, ctas, st);
+    default: return launch_kind<64, 1>(kind, mA, mB, mB128, g, ctas, st);
   }
 }
 
@@ -1352,19 +1388,17 @@ static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
 }
 
 // Split lists the workspace must hold for any batch height up to rows_cap.
-static size_t lists_needed(int rows_cap, int n_tiles, int ctas, int forced, int mode, int KT) {
+static size_t lists_needed(int rows_cap, long long N, int ctas, int forced, int mode, int KT) {
   size_t lists = 0;
-  for (int nb = BM; nb < rows_cap + BM; nb += BM) {
-    int h = nb < rows_cap ? nb : rows_cap;
-    int kind = kernel_kind(mode, h);
-    int tile = kind == 2 ? 256 : BM;
-    int mt = (h + tile - 1) / tile;
-    int c = kind == 2 ? (ctas / 2 > 0 ? ctas / 2 : 1) : ctas;
-    // either kernel may leave two partial lists per row and split
-    (void)kind;
-    const int H = KT <= 32 ? 2 : 1;
-    size_t l = (size_t)choose_splits(mt, n_tiles, c, forced, MAX_LISTS / H, kind == 2, KT) * H * mt * tile;
-    if (l > lists) lists = l;
+  const int H = KT <= 32 ? 2 : 1;  // either kernel may leave two partial lists per row and split
+  for (int nb = 1; nb < rows_cap + BM; nb = nb == 1 ? BM : nb + BM) {
+    const int h = nb < rows_cap ? nb : rows_cap;
+    const int kind = kernel_kind(mode, h);
+    const int tile = kind == 2 ? 256 : BM;
+    const int mt = (h + tile - 1) / tile;
+    const int c = kind == 2 ? (ctas / 2 > 0 ? ctas / 2 : 1) : ctas;
+    const ColumnPlan p = plan_columns(N, h, mt, c, forced, MAX_LISTS / H, kind == 2, KT);
+    lists = std::max(lists, (size_t)p.splits * H * mt * tile);
   }
   return lists;
 }
@@ -1384,7 +1418,6 @@ struct r2m_engine {
   int score_mode;
   int ctas;
   int forced_splits;
-  int n_tiles;
   CUtensorMap mapB;
   CUtensorMap mapB128;  // 128-row box for the CTA-pair kernel
   int mode;             // 0 auto, 1 single-CTA kernel, 2 CTA-pair kernel
@@ -1446,7 +1479,6 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
       }
     }
   }
-  e->n_tiles = (int)((N + BN - 1) / BN);
   rc = make_map(&e->mapB, d_B, N, rdim, BN);
   if (!rc) rc = make_map(&e->mapB128, d_B, N, rdim, 128);
   if (rc) {
@@ -1454,7 +1486,7 @@ extern "C" int r2m_engine_create(const uint8_t *d_B, const float *d_scaleB, int 
     return rc;
   }
   // workspace: the largest (read tiles x splits) any batch height can ask for
-  size_t lists = lists_needed(rows_cap, e->n_tiles, e->ctas, e->forced_splits, e->mode, e->KT);
+  size_t lists = lists_needed(rows_cap, N, e->ctas, e->forced_splits, e->mode, e->KT);
   e->part_lists = lists;
   if (alloc_workspace(lists, e->KT, &e->ws) != cudaSuccess) {
     delete e;
@@ -1487,7 +1519,7 @@ extern "C" int r2m_engine_set_tuning(r2m_engine *eng, const r2m_tuning *tune) {
   const int forced = tune->splits > 0 ? tune->splits : 0;
   const int mode = (tune->reserved[1] >= 0 && tune->reserved[1] <= 2) ? tune->reserved[1] : 0;
   const int KT = kt_for(eng->k, tune);
-  size_t lists = lists_needed(eng->rows_cap, eng->n_tiles, ctas, forced, mode, KT);
+  size_t lists = lists_needed(eng->rows_cap, eng->N_cap, ctas, forced, mode, KT);
   if (lists * KT > eng->part_lists * eng->KT) {  // grow the split workspace
     Workspace w;
     if (alloc_workspace(lists, KT, &w) != cudaSuccess)
@@ -1532,7 +1564,6 @@ int engine_rebind(r2m_engine *eng, const uint8_t *d_B, const float *d_scaleB, in
   eng->B = d_B;
   eng->scaleB = d_scaleB;
   eng->N = N;
-  eng->n_tiles = (int)((N + BN - 1) / BN);
   eng->mapB = m;
   eng->mapB128 = m128;
   return R2M_OK;
@@ -1574,15 +1605,20 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.nb = nb;
   g.num_m_tiles = (nb + tile - 1) / tile;
   g.N = eng->N;
-  g.n_tiles = eng->n_tiles;
   const int hmax = eng->KT <= 32 ? 2 : 1;
   // (a rebound index of fewer columns may prefer more splits than the
   // workspace was sized for)
   const size_t room = eng->part_lists / ((size_t)hmax * g.num_m_tiles * tile);
-  g.splits = choose_splits(g.num_m_tiles, eng->n_tiles, ctas_eff, eng->forced_splits,
-                           (int)std::min<size_t>(MAX_LISTS / hmax, room), kind == 2, eng->KT);
+  const ColumnPlan plan =
+      plan_columns(eng->N, nb, g.num_m_tiles, ctas_eff, eng->forced_splits,
+                   (int)std::min<size_t>(MAX_LISTS / hmax, room), kind == 2, eng->KT, eng->epi != 1 || hmax == 1);
+  g.bn = plan.bn;
+  g.n_tiles = plan.n_tiles;
+  g.splits = plan.splits;
+  CUtensorMap narrow;
+  if (plan.bn != BN && (rc = make_map(&narrow, eng->B, eng->N, eng->rdim, kind == 2 ? plan.bn / 2 : plan.bn))) return rc;
   const int halves =
-      eng->epi == 1 ? 1 : eng->epi == 2 ? hmax : epi_halves_for(kind, eng->KT, eng->n_tiles, g.splits);
+      eng->epi == 1 ? 1 : eng->epi == 2 ? hmax : epi_halves_for(kind, eng->KT, g.n_tiles, g.splits);
   const int lists_per_row = halves * g.splits;  // partial lists each row leaves
   g.num_kb = (eng->rdim + BK - 1) / BK;
   g.score_mode = eng->score_mode;
@@ -1610,7 +1646,8 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
     R2M_CUDA(cudaMemsetAsync(eng->ws.pace, 0, kPaceSlots * sizeof(long long) + eng->pub_lists * sizeof(uint32_t), st));
   eng->dirty = true;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[0], st));
-  rc = dispatch_gemm(kind, halves, eng->KT, mapA, eng->mapB, eng->mapB128, g, ctas, st);
+  rc = dispatch_gemm(kind, halves, eng->KT, mapA, plan.bn != BN ? narrow : eng->mapB,
+                     plan.bn != BN ? narrow : eng->mapB128, g, ctas, st);
   if (rc) return rc;
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[1], st));
   if ((rc = launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, ctas, st))) return rc;
@@ -1757,16 +1794,16 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   int rc = noalloc_setup(&scratch, &err);
   if (rc) return rc;
   cudaStream_t st = as_stream(stream);
-  CUtensorMap mapA, mapB, mapB128;
-  if ((rc = make_map(&mapB, d_B, N, rdim, BN))) return rc;
-  if ((rc = make_map(&mapB128, d_B, N, rdim, 128))) return rc;
-  if ((rc = make_map(&mapA, d_A, nb, rdim, BM))) return rc;
-  const int n_tiles = (int)((N + BN - 1) / BN);
   const int sms = sm_count();
   const int ctas_eff = kind == 2 ? (sms / 2 > 0 ? sms / 2 : 1) : sms;
   const int hmax = KT <= 32 ? 2 : 1;
   // the engine's automatic schedule, with the splits cut to the scratch
-  int splits = choose_splits(m_tiles, n_tiles, ctas_eff, 0, MAX_LISTS / hmax, kind == 2, KT);
+  const ColumnPlan plan = plan_columns(N, nb, m_tiles, ctas_eff, 0, MAX_LISTS / hmax, kind == 2, KT);
+  CUtensorMap mapA, mapB;
+  if ((rc = make_map(&mapB, d_B, N, rdim, kind == 2 ? plan.bn / 2 : plan.bn))) return rc;
+  if ((rc = make_map(&mapA, d_A, nb, rdim, BM))) return rc;
+  const int n_tiles = plan.n_tiles;
+  int splits = plan.splits;
   int halves = epi_halves_for(kind, KT, n_tiles, splits);
   while (splits > 1 && (size_t)halves * splits * mpad > max_lists) {
     --splits;
@@ -1777,6 +1814,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
   g.nb = nb;
   g.num_m_tiles = m_tiles;
   g.N = N;
+  g.bn = plan.bn;
   g.n_tiles = n_tiles;
   g.splits = splits;
   g.num_kb = (rdim + BK - 1) / BK;
@@ -1809,7 +1847,7 @@ extern "C" int r2m_batch_gemm_topk_noalloc(const uint8_t *d_B, const float *d_sc
     g.pub = reinterpret_cast<uint32_t *>(lists + nlists * list_bytes);
     R2M_CUDA(cudaMemsetAsync(g.pub, 0, nlists * sizeof(uint32_t), st));
   }
-  rc = dispatch_gemm(kind, halves, KT, mapA, mapB, mapB128, g, ctas, st);
+  rc = dispatch_gemm(kind, halves, KT, mapA, mapB, mapB, g, ctas, st);
   if (rc) return rc;
   if ((rc = launch_merge(g, halves * splits, KT, d_scaleA, d_vals, d_locs, ctas, st))) return rc;
   k_noalloc_poison<<<64, 256, 0, st>>>(err, d_vals, d_locs, (long long)nb * k);

@@ -22,10 +22,7 @@ def levels(order, N):
             "saw": 1 + (j * 37 % 113) + (j // 113) % 100}[order]
 
 
-@pytest.mark.parametrize("order", ["rising", "falling", "flat", "saw"])
-@pytest.mark.parametrize("nb,N,splits", [(1, 64, 0), (37, 511, 1), (128, 2305, 0), (129, 2305, 2), (300, 4097, 3)])
-@pytest.mark.parametrize("k,score", [(1, "f32"), (5, "f16"), (16, "scaled"), (20, "f16"), (32, "scaled"), (64, "f32")])
-def test_every_candidate_order(order, nb, N, splits, k, score):
+def check(order, nb, N, splits, k, score):
     lv = levels(order, N)
     B = (np.arange(RDIM)[None, :] < lv[:, None]).astype(np.uint8) * ONE
     # row r sees the first RDIM - r % 97 levels: equal scores beyond, other thresholds
@@ -49,3 +46,19 @@ def test_every_candidate_order(order, nb, N, splits, k, score):
         assert np.array_equal(l.cpu().numpy(), loc + 1)
         assert np.array_equal(v.cpu().numpy(), val)
         eng.close()
+
+
+@pytest.mark.parametrize("order", ["rising", "falling", "flat", "saw"])
+@pytest.mark.parametrize("nb,N,splits", [(1, 64, 0), (37, 511, 1), (128, 2305, 0), (129, 2305, 2), (300, 4097, 3)])
+@pytest.mark.parametrize("k,score", [(1, "f32"), (5, "f16"), (16, "scaled"), (20, "f16"), (32, "scaled"), (64, "f32")])
+def test_every_candidate_order(order, nb, N, splits, k, score):
+    check(order, nb, N, splits, k, score)
+
+
+# sizes at which units are one or two tiles: 64, 128, 192 and 256 columns wide
+@pytest.mark.parametrize("order", ["rising", "saw"])
+@pytest.mark.parametrize("nb", [1, 16, 128, 129, 256, 1000])
+@pytest.mark.parametrize("N", [65, 1000, 4736, 9473, 14209, 20000])
+@pytest.mark.parametrize("k,score", [(20, "scaled"), (64, "f16")])
+def test_few_columns_per_unit(order, nb, N, k, score):
+    check(order, nb, N, 0, k, score)
