@@ -842,6 +842,13 @@ __device__ __forceinline__ void st_planes(float2 *base, int stride, int i, const
   }
 }
 
+// The reference's norm of a row of energy e: sqrt(e) + 1e-16 in fp64, which
+// rounds back to the root from 1e-8 up.
+__device__ __forceinline__ float norm_of(float e) {
+  const float root = sqrtf(e);
+  return root >= 1e-8f ? root : (float)((double)root + 1e-16);
+}
+
 // Sum each of M values over the warp into every lane: the xor butterfly's
 // sums (offsets 16, 8, 4, 2, 1), but the lanes split the values between them
 // while there are several, so M = 4 takes 10 shuffles instead of 20 (with the
@@ -994,9 +1001,7 @@ __device__ __forceinline__ void sparse_fragment(const EncParams &P, const float2
     tot += part[q];
     mine = lane == q ? part[q] : mine;
   }
-  // sqrt + 1e-16 in fp64; from 1e-8 up the sum rounds back to the root
-  const float root = sqrtf(tot);
-  const float nrm = root >= 1e-8f ? root : (float)((double)root + 1e-16);
+  const float nrm = norm_of(tot);
   if (lane < M) norms_out[lane] = lane == 0 ? nrm : mine;
   // x / nrm for every value with one reciprocal: y = RN(1/nrm), q0 = x*y,
   // r = x - q0*nrm (exact with FMA), RN(q0 + r*y) is the correctly rounded
@@ -1862,8 +1867,8 @@ __global__ void __launch_bounds__(128) k_rescore_fp32(EncParams P, const uint32_
 // read, the candidates dealt out to its warps.  What bounds it is instruction
 // issue: a candidate is a whole encode (nw windows) and a dot product over
 // every bin, against a few hundred bytes of memory traffic.  So
-//   * a lane's 2T embedding values of the read (bins lane + 32 t) stay in its
-//     registers for all candidates;
+//   * the read's embedding is formed once per block, in shared memory: kept
+//     in registers by every warp, its 64 values held the SM to 12 warps;
 //   * the dot product divides with the encoder's reciprocal + FMA correction
 //     (the correctly rounded x / nrm) on (Re, Im) pairs;
 //   * window groups come from shared lane masks and are added in rounds, as
@@ -1871,7 +1876,7 @@ __global__ void __launch_bounds__(128) k_rescore_fp32(EncParams P, const uint32_
 //     cost less here than slots looked up per bin;
 //   * the ranks of the candidates are counted by all lanes.
 // 4,000 reads x 64 candidates of 150 bases (s8 m4 c4): 3,900 us with the general
-// kernel, 774 us with this one.
+// kernel, 652 us with this one.
 // Every sum is formed in the general kernel's order (bins in window order, the
 // energies along float4 slots, the dot product over bins lane + 32 t, Re
 // before Im), so the scores are the same bits.
@@ -1892,9 +1897,9 @@ __device__ __forceinline__ float rescore_hist(const EncParams &P, const float2 *
     const bool valid = p < nw;
     const int wo = p >> 4;
     const uint32_t w0 = __shfl_sync(FULL, wreg, wo & 31), w1 = __shfl_sync(FULL, wreg, (wo + 1) & 31);
-    const uint32_t smer = __funnelshift_r(w0, w1, (uint32_t)(p & 15) << 1) & bmask;
+    const uint32_t smer = __funnelshift_r(w0, w1, (uint32_t)(lane & 15) << 1) & bmask;
     const uint32_t upper = c2 >= 32u ? 0u : (smer >> c2);
-    const uint32_t cb = (smer & cbmask) ^ ((upper * 0x9E3779B1u) & cbmask);
+    const uint32_t cb = (smer ^ (upper * 0x9E3779B1u)) & cbmask;
     if (valid) atomicOr(gmask + cb, 1u << lane);
     __syncwarp();
     const unsigned grp = valid ? gmask[cb] : (1u << lane);
@@ -1940,24 +1945,16 @@ __device__ __forceinline__ float rescore_hist(const EncParams &P, const float2 *
       a1 += e1;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 += __shfl_xor_sync(FULL, a0, o);
-    a1 += __shfl_xor_sync(FULL, a1, o);
-    a2 += __shfl_xor_sync(FULL, a2, o);
-    a3 += __shfl_xor_sync(FULL, a3, o);
-  }
+  float part[4] = {a0, a1, a2, a3};
+  warp_sums<4>(part);
   float tot;
-  if constexpr (M == 4) tot = ((a0 + a1) + a2) + a3;
-  else if constexpr (M == 2) tot = (a0 + a2) + (a1 + a3);
-  else tot = (a0 + a2) + (a1 + a3);
-  return (float)((double)sqrtf(tot) + 1e-16);
+  if constexpr (M == 4) tot = ((part[0] + part[1]) + part[2]) + part[3];
+  else tot = (part[0] + part[2]) + (part[1] + part[3]);
+  return norm_of(tot);
 }
 
-constexpr int kRescoreWarps = 4;
-
-template <int M, int T>
-__global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
+template <int M, int T, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) k_rescore_dense(
     EncParams P, const uint32_t *__restrict__ dnas, int nb, const int *__restrict__ cand, int kc,
     const uint32_t *__restrict__ genome, const int64_t *__restrict__ col_pos, const uint8_t *__restrict__ strand,
     long long N, float *scores, float *out_v, int *out_l, int k) {
@@ -1968,7 +1965,8 @@ __global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
   float2 *table = reinterpret_cast<float2 *>(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
-  float *hist = reinterpret_cast<float *>(smem + sparse_table_bytes(P)) + warp * (64 * T + NCM);
+  float *emb = reinterpret_cast<float *>(smem + sparse_table_bytes(P));
+  float *hist = emb + 64 * T + warp * (64 * T + NCM);
   uint32_t *gmask = reinterpret_cast<uint32_t *>(hist + 64 * T);
   for (int i = lane; i < NCM; i += 32) gmask[i] = 0u;
   sparse_table(P, table);  // ends with a block barrier
@@ -1976,22 +1974,23 @@ __global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
   const uint32_t tailmask = rr == 0 ? 0xFFFFFFFFu : ((1u << (2 * rr)) - 1u);
   const uint32_t shbits = (uint32_t)(32 * W - 2 * P.k);
   for (int row = blockIdx.x; row < nb; row += gridDim.x) {
-    // the read's embedding: values of bins lane + 32 t
-    float2 emb[T];
-    {
+    // the read's embedding, by warp 0: values of bins lane + 32 t
+    if (warp == 0) {
       const uint32_t wreg = lane < W ? __ldg(dnas + (size_t)row * W + lane) : 0u;
       const float nrm = rescore_hist<M, T>(P, table, hist, gmask, wreg);
       const float y = __frcp_rn(nrm);
       const float2 y2 = make_float2(y, y), nn2 = make_float2(-nrm, -nrm);
-#pragma unroll
+#pragma unroll 4
       for (int t = 0; t < T; ++t) {
         const float2 x = *reinterpret_cast<const float2 *>(hist + hoff(lane + 32 * t));
         const float2 q0 = mul2(x, y2);
-        emb[t] = fma2(fma2(q0, nn2, x), y2, q0);
+        const float2 d = fma2(fma2(q0, nn2, x), y2, q0);
+        emb[lane + 32 * t] = d.x;
+        emb[32 * T + lane + 32 * t] = d.y;
       }
-      __syncwarp();
     }
-    for (int j = warp; j < kc; j += kRescoreWarps) {
+    __syncthreads();
+    for (int j = warp; j < kc; j += WARPS) {
       const int c1 = __ldg(cand + (size_t)row * kc + j);
       float s = -INFINITY;
       if (c1 >= 1 && c1 <= N) {
@@ -2007,17 +2006,18 @@ __global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
         if (__ldg(strand + col)) wreg = revcomp_reg(wreg, W, shbits);
         const float nrm = rescore_hist<M, T>(P, table, hist, gmask, wreg);
         const float y = __frcp_rn(nrm);
-        float acc = 0.f;
+        const float2 y2 = make_float2(y, y), nn2 = make_float2(-nrm, -nrm);
+        float acc = 0.f, im[T];
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-          const float x = hist[hoff(lane + 32 * t)], q0 = x * y;
-          acc = fmaf(emb[t].x, fmaf(fmaf(-q0, nrm, x), y, q0), acc);
+          const float2 x = *reinterpret_cast<const float2 *>(hist + hoff(lane + 32 * t));
+          const float2 q0 = mul2(x, y2);
+          const float2 d = fma2(fma2(q0, nn2, x), y2, q0);
+          acc = fmaf(emb[lane + 32 * t], d.x, acc);
+          im[t] = d.y;
         }
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-          const float x = hist[hoff(lane + 32 * t) + 1], q0 = x * y;
-          acc = fmaf(emb[t].y, fmaf(fmaf(-q0, nrm, x), y, q0), acc);
-        }
+        for (int t = 0; t < T; ++t) acc = fmaf(emb[32 * T + lane + 32 * t], im[t], acc);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
         s = acc;
@@ -2049,20 +2049,31 @@ __global__ void __launch_bounds__(32 * kRescoreWarps, 3) k_rescore_dense(
   }
 }
 
+template <int M, int T, int WARPS>
+static int launch_rescore_as(const EncParams &P, const uint32_t *dnas, int nb, const int *cand, int kc,
+                          const uint32_t *genome, const int64_t *col_pos, const uint8_t *strand, long long N,
+                          float *scores, float *out_v, int *out_l, int k, cudaStream_t st) {
+  auto kern = k_rescore_dense<M, T, WARPS>;
+  const size_t smem = sparse_table_bytes(P) + (size_t)(WARPS * (64 * T + 32 * T / M) + 64 * T) * 4;
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 1;
+  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS, smem));
+  const long long cap = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
+  kern<<<(unsigned)(nb < cap ? nb : cap), 32 * WARPS, smem, st>>>(P, dnas, nb, cand, kc, genome, col_pos,
+                                                                         strand, N, scores, out_v, out_l, k);
+  R2M_CUDA(cudaGetLastError());
+  return R2M_OK;
+}
+
+// Four warps per read; eight where there are fewer reads than they would fill
+// the SMs with (100 reads x 20 candidates: 35.0 -> 29.0 us).
 template <int M, int T>
 static int launch_rescore(const EncParams &P, const uint32_t *dnas, int nb, const int *cand, int kc,
                           const uint32_t *genome, const int64_t *col_pos, const uint8_t *strand, long long N,
                           float *scores, float *out_v, int *out_l, int k, cudaStream_t st) {
-  auto kern = k_rescore_dense<M, T>;
-  const size_t smem = sparse_table_bytes(P) + (size_t)kRescoreWarps * (64 * T + 32 * T / M) * 4;
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 1;
-  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kRescoreWarps, smem));
-  const long long cap = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
-  kern<<<(unsigned)(nb < cap ? nb : cap), 32 * kRescoreWarps, smem, st>>>(P, dnas, nb, cand, kc, genome, col_pos,
-                                                                         strand, N, scores, out_v, out_l, k);
-  R2M_CUDA(cudaGetLastError());
-  return R2M_OK;
+  if (nb <= 2 * sm_count())
+    return launch_rescore_as<M, T, 8>(P, dnas, nb, cand, kc, genome, col_pos, strand, N, scores, out_v, out_l, k, st);
+  return launch_rescore_as<M, T, 4>(P, dnas, nb, cand, kc, genome, col_pos, strand, N, scores, out_v, out_l, k, st);
 }
 
 }  // namespace r2m
