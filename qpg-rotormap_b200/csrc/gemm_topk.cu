@@ -76,7 +76,7 @@ struct GemmArgs {
   int num_kb;
   int score_mode;
   int k;     // results wanted per row (<= KT)
-  int mpad;  // num_m_tiles * BM (partial-list row stride)
+  int mpad;  // partial-list row stride, at least nb
   const float *scaleB;
   float *part_vals;
   int *part_cols;
@@ -1362,8 +1362,8 @@ static int bound_splits(int ctas, int m_tiles, int splits, int halves) {
 }
 
 // One allocation: the pacing slots and the row bounds (zero between launches),
-// then `lists` partial lists of KT values and columns.  The lists come in
-// tiles of 128, which keeps every part 16-byte aligned.
+// then `lists` partial lists of KT values and columns.  `lists` is a multiple
+// of 8, which keeps every part 16-byte aligned.
 struct Workspace {
   long long *pace;
   uint32_t *pub;
@@ -1387,6 +1387,10 @@ static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   return cudaSuccess;
 }
 
+// Rows of a partial list (its stride): the batch, rounded up so that the parts
+// of the workspace stay aligned.
+static int list_rows(int nb) { return (nb + 7) & ~7; }
+
 // Split lists the workspace must hold for any batch height up to rows_cap.
 static size_t lists_needed(int rows_cap, long long N, int ctas, int forced, int mode, int KT) {
   size_t lists = 0;
@@ -1398,7 +1402,7 @@ static size_t lists_needed(int rows_cap, long long N, int ctas, int forced, int 
     const int mt = (h + tile - 1) / tile;
     const int c = kind == 2 ? (ctas / 2 > 0 ? ctas / 2 : 1) : ctas;
     const ColumnPlan p = plan_columns(N, h, mt, c, forced, MAX_LISTS / H, kind == 2, KT);
-    lists = std::max(lists, (size_t)p.splits * H * mt * tile);
+    lists = std::max(lists, (size_t)p.splits * H * list_rows(h));
   }
   return lists;
 }
@@ -1608,7 +1612,7 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   const int hmax = eng->KT <= 32 ? 2 : 1;
   // (a rebound index of fewer columns may prefer more splits than the
   // workspace was sized for)
-  const size_t room = eng->part_lists / ((size_t)hmax * g.num_m_tiles * tile);
+  const size_t room = eng->part_lists / ((size_t)hmax * list_rows(nb));
   const ColumnPlan plan =
       plan_columns(eng->N, nb, g.num_m_tiles, ctas_eff, eng->forced_splits,
                    (int)std::min<size_t>(MAX_LISTS / hmax, room), kind == 2, eng->KT, eng->epi != 1 || hmax == 1);
@@ -1623,7 +1627,7 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   g.num_kb = (eng->rdim + BK - 1) / BK;
   g.score_mode = eng->score_mode;
   g.k = eng->k;
-  g.mpad = g.num_m_tiles * tile;
+  g.mpad = list_rows(nb);
   g.scaleB = eng->scaleB;
   g.part_vals = eng->ws.vals;
   g.part_cols = eng->ws.cols;
