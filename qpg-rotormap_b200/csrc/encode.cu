@@ -15,8 +15,9 @@
 //   * normalize modes 0..3 as the reference; the real row is the split
 //     [Re(bin 0..D-1); Im(bin 0..D-1)], D = m*4^c.
 //
-// B200 design: one warp per fragment (the reference spends one 512-thread
-// block per 150-base read with 143 active threads).  The phasor of every
+// B200 design: one warp per fragment at read length (the reference spends one
+// 512-thread block per 150-base read with 143 active threads), one block per
+// long fragment.  The phasor of every
 // (idm, p) is computed once per block into shared memory with the exact fp32
 // recipe of the reference thread that owns window p (direct cos/sin at the
 // thread's first window, then the fp32 complex recurrence), so the values
@@ -713,13 +714,32 @@ template <>
 struct Bytes<8> { using T = uint2; };
 template <>
 struct Bytes<16> { using T = uint4; };
-// A Re run and an Im run side by side: one shared-memory access up to 16 bytes.
-// The output pass looks a c-mer up once for both of its chunks (apart, twice:
-// 1,000,000 index columns at m = 4 1,611 -> 1,506 us, 65,536 reads at m = 1
-// 111.9 -> 97.7).
+// The converted runs of the slots.  Up to 8 bytes a run, Re and Im lie side by
+// side, one shared-memory access for both: the output pass looks a c-mer up
+// once for its two chunks (apart, twice: 1,000,000 index columns at m = 4 1,611
+// -> 1,506 us, 65,536 reads at m = 1 111.9 -> 97.7).  Runs of 16 bytes stay in
+// two planes: pairs of them would start on every other bank group only.
 template <typename T>
-struct __align__(sizeof(T) <= 8 ? 2 * sizeof(T) : 16) RunPair {
-  T re, im;
+struct Runs {
+  static constexpr bool PAIR = sizeof(T) <= 8;
+  struct __align__(PAIR ? 2 * sizeof(T) : 16) Two {
+    T re, im;
+  };
+  T *base;
+  int plane;  // slots
+
+  __device__ __forceinline__ void put(int sl, T re, T im) const {
+    if constexpr (PAIR) {
+      reinterpret_cast<Two *>(base)[sl] = Two{re, im};
+    } else {
+      base[sl] = re;
+      base[plane + sl] = im;
+    }
+  }
+  __device__ __forceinline__ Two get(int sl) const {
+    if constexpr (PAIR) return reinterpret_cast<const Two *>(base)[sl];
+    else return Two{base[sl], base[plane + sl]};
+  }
 };
 
 __device__ __forceinline__ unsigned long long f2_bits(float2 a) {
@@ -894,7 +914,7 @@ __device__ __forceinline__ void sparse_fragment(const EncParams &P, const float2
   const int ns = P.sp_nslot;  // entries per accumulator plane
   uint8_t *smap = warea;
   float2 *acc = reinterpret_cast<float2 *>(warea + L.smap);
-  RunPair<T> *conv = reinterpret_cast<RunPair<T> *>(warea + L.smap + L.acc);
+  const Runs<T> conv = {reinterpret_cast<T *>(warea + L.smap + L.acc), ns};
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xFFFFFFFFu;
   const unsigned lt = (1u << lane) - 1u;
@@ -902,7 +922,7 @@ __device__ __forceinline__ void sparse_fragment(const EncParams &P, const float2
   // group masks of the accumulation: bit l of gmask[cb] = lane l's window
   // has c-mer cb (formed with shared atomic ORs, cleared by each group's
   // leader after its batch, so zero between batches)
-  uint32_t *gmask = reinterpret_cast<uint32_t *>(conv);
+  uint32_t *gmask = reinterpret_cast<uint32_t *>(conv.base);
   for (int i = lane * 16; i < ncm; i += 512) *reinterpret_cast<uint4 *>(smap + i) = make_uint4(~0u, ~0u, ~0u, ~0u);
   for (int i = lane * 4; i < ncm; i += 128) *reinterpret_cast<uint4 *>(gmask + i) = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
@@ -1032,7 +1052,7 @@ __device__ __forceinline__ void sparse_fragment(const EncParams &P, const float2
       re[q] = d.x;
       im[q] = d.y;
     }
-    conv[sl] = RunPair<T>{pack_part<OUT, M>(re), pack_part<OUT, M>(im)};
+    conv.put(sl, pack_part<OUT, M>(re), pack_part<OUT, M>(im));
   }
   __syncwarp();
   // ---- the dense row, 16-byte chunks, c-mer-major: [Re part | Im part], the
@@ -1050,9 +1070,9 @@ __device__ __forceinline__ void sparse_fragment(const EncParams &P, const float2
     } re, im;
 #pragma unroll
     for (int e = 0; e < CPC; ++e) {
-      RunPair<T> val = {T(), T()};
+      typename Runs<T>::Two val = {T(), T()};
       const int sl = sm.b[e];
-      if (sl != 0xFF) val = conv[sl];
+      if (sl != 0xFF) val = conv.get(sl);
       re.t[e] = val.re;
       im.t[e] = val.im;
     }
@@ -1080,16 +1100,20 @@ __host__ __device__ inline size_t sparse_table_bytes(const EncParams &P) {
   return ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
 }
 
-// Warps per block, by the copies m.  Shared memory bounds the residency (a
-// warp's area is about 6 KB at m = 4, the phasor table 4.5 KB a block at 150
-// bases): at m = 4 two blocks of 18 warps per SM share two tables where four of
-// 8 warps held four, 36 warps instead of 32.  65,536 reads of 150 bases 119.1
-// -> 114.5 us, of 250 bases 206 -> 186; 1,000,000 index columns of 150 bases
-// 1,694 -> 1,613 us, 200,000 of 250 bases 614 -> 533.
-__host__ __device__ constexpr int sparse_warps(int m) { return m == 4 ? 18 : 8; }
+// Warps per block.  Shared memory bounds the residency of the one-byte forms at
+// m = 4 (a warp's area is about 6 KB, the phasor table 4.5 KB a block at 150
+// bases): two blocks of 18 warps per SM share two tables where four of 8 warps
+// held four, 36 warps instead of 32.  65,536 reads of 150 bases 119.1 -> 114.5
+// us, of 250 bases 206 -> 186; 1,000,000 index columns of 150 bases 1,694 ->
+// 1,613 us, 200,000 of 250 bases 614 -> 533.  The wider forms need the registers
+// that 36 warps leave them too few of (20,000 reads of 60 bases to fp16 27.2 us
+// with 18 warps, 23.3 with 8).
+__host__ __device__ constexpr int sparse_warps(int m, int outb) { return m == 4 && outb == 1 ? 18 : 8; }
 
 template <int OUT, int M>
-__global__ void __launch_bounds__(32 * sparse_warps(M), M == 4 ? 2 : M < 4 ? 4 : 1) k_encode_sparse(EncParams P, const uint32_t *__restrict__ dnas, int64_t n,
+__global__ void __launch_bounds__(32 * sparse_warps(M, OutT<OUT>::bytes),
+                                  sparse_warps(M, OutT<OUT>::bytes) == 18 ? 2 : M < 4 ? 4 : 1)
+    k_encode_sparse(EncParams P, const uint32_t *__restrict__ dnas, int64_t n,
                                                        void *dest, float *norms, float *scales) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2 *table = reinterpret_cast<float2 *>(smem);
@@ -1111,7 +1135,9 @@ __global__ void __launch_bounds__(32 * sparse_warps(M), M == 4 ? 2 : M < 4 ? 4 :
 }
 
 template <int OUT, int M>
-__global__ void __launch_bounds__(32 * sparse_warps(M), M == 4 ? 2 : M < 4 ? 4 : 1) k_encode_sparse_ref(EncParams P, const uint32_t *__restrict__ genome,
+__global__ void __launch_bounds__(32 * sparse_warps(M, OutT<OUT>::bytes),
+                                  sparse_warps(M, OutT<OUT>::bytes) == 18 ? 2 : M <= 4 ? 4 : 1)
+    k_encode_sparse_ref(EncParams P, const uint32_t *__restrict__ genome,
                                                            const int64_t *__restrict__ win_pos, int64_t nwin,
                                                            int64_t batch, void *dest, float *norms,
                                                            float *scales) {
@@ -1488,14 +1514,14 @@ template <typename KernelFn>
 static int sparse_grid(KernelFn kern, const EncParams &P, int outb, int64_t nwork, int *grid, int *block,
                        size_t *smem) {
   const SparseLayout L = sparse_layout(P.c, P.m, P.sp_nslot, outb);
-  // as many warps as fit, at m = 4 in two blocks per SM unless one larger block
-  // holds more
+  // as many warps as fit, blocks of 18 two per SM unless one larger block holds
+  // more
   const size_t tb = sparse_table_bytes(P), most = 200 * 1024, half = 113 * 1024;
   auto fit = [&](size_t bytes) {
-    return bytes > tb ? (int)std::min<size_t>(sparse_warps(P.m), (bytes - tb) / L.warp) : 0;
+    return bytes > tb ? (int)std::min<size_t>(sparse_warps(P.m, outb), (bytes - tb) / L.warp) : 0;
   };
   int wpb = fit(most);
-  if (P.m == 4 && 2 * fit(half) >= wpb) wpb = fit(half);
+  if (sparse_warps(P.m, outb) == 18 && 2 * fit(half) >= wpb) wpb = fit(half);
   // few fragments: blocks of 8 warps reach more SMs (1,000 reads of 150 bases
   // 12.7 -> 11.7 us, the host's share of a call)
   const int64_t spread = (nwork + sm_count() - 1) / sm_count();
