@@ -1528,7 +1528,9 @@ static int sparse_grid(KernelFn kern, const EncParams &P, int outb, int64_t nwor
   wpb = std::max(1, std::min(wpb, (int)std::max<int64_t>(spread, 8)));
   *block = 32 * wpb;
   *smem = sparse_table_bytes(P) + (size_t)L.warp * wpb;
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+  // the limit is per function, not per launch: the same for every caller, so that
+  // threads encoding with other sizes do not lower it
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   int per_sm = 0;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, *block, *smem));
   if (per_sm < 1) per_sm = 1;
@@ -1570,6 +1572,8 @@ static int launch_sparse_ref(const EncParams &P, void *dest, float *norms, float
   }
 }
 
+constexpr int kLongSmem = 220 * 1024;  // most shared memory of a block (the limit set for every launch)
+
 // Window tile of the block-per-fragment path for `items` fragments, 0 where
 // the one-warp path is the faster one (or the tile does not fit shared memory:
 // over 1,024 c-mers with m > 4).  A block's fragment takes about 4 us and 6 us
@@ -1582,8 +1586,8 @@ static int long_tile(const EncParams &P, int64_t items) {
   const char *force = getenv("R2M_ENCODER");
   if (force && strcmp(force, "dense") == 0) return 0;
   if (P.nw <= 512) return 0;
-  int tile = P.m <= 2 && long_layout(P, 4096).total <= 220 * 1024 ? 4096 : 0;
-  if (tile == 0 && long_layout(P, 2048).total <= 220 * 1024) tile = 2048;
+  int tile = P.m <= 2 && long_layout(P, 4096).total <= kLongSmem ? 4096 : 0;
+  if (tile == 0 && long_layout(P, 2048).total <= kLongSmem) tile = 2048;
   if (tile == 0) return 0;
   const double sms = sm_count();
   const double block_us = std::ceil(items / (2 * sms)) * (4.0 + 6.0 * ((P.nw + tile - 1) / tile));
@@ -1596,7 +1600,7 @@ static int launch_long_as(const EncParams &P, const uint32_t *src, const int64_t
                           int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
   auto kern = k_encode_long<OUT, TW, REF>;
   const int smem = long_layout(P, TW).total;
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem));
   int per_sm = 1;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLongThreads, smem));
   const int64_t cap = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
@@ -2084,7 +2088,7 @@ static int launch_rescore_as(const EncParams &P, const uint32_t *dnas, int nb, c
                           float *scores, float *out_v, int *out_l, int k, cudaStream_t st) {
   auto kern = k_rescore_dense<M, T, WARPS>;
   const size_t smem = sparse_table_bytes(P) + (size_t)(WARPS * (64 * T + 32 * T / M) + 64 * T) * 4;
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
   int per_sm = 1;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * WARPS, smem));
   const long long cap = (long long)sm_count() * (per_sm > 0 ? per_sm : 1);
