@@ -10,7 +10,9 @@
  *   - `stream` is a cudaStream_t (NULL = the legacy default stream); every
  *     device call is stream-ordered and returns without synchronizing unless
  *     its comment says otherwise (the device FASTA reader learns its record
- *     counts on the host; destroying an engine waits for its work);
+ *     counts on the host; creating an engine waits until its workspace is
+ *     cleared, so that the first search may come on any stream; destroying an
+ *     engine waits for its work);
  *   - an engine or reader handle serves one thread at a time (its workspace,
  *     events and rebound tensor maps are per handle); different handles may
  *     be used from different threads and streams concurrently;

@@ -1375,7 +1375,14 @@ static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   const size_t part = lists * KT * sizeof(float), zero = kPaceSlots * sizeof(long long) + lists * sizeof(uint32_t);
   cudaError_t e = cudaMalloc(&p, zero + 2 * part);
   if (e != cudaSuccess) return e;
-  e = cudaMemset(p, 0, zero);
+  // The first search may come at once and on any stream, and recycled memory
+  // read as row bounds drops results: the zeros are in place before this
+  // returns.  A stream of its own, so that work queued elsewhere is not waited for.
+  cudaStream_t st = nullptr;
+  e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, zero, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (st) cudaStreamDestroy(st);
   if (e != cudaSuccess) {
     cudaFree(p);
     return e;

@@ -1,0 +1,52 @@
+"""The state an engine keeps between searches (row bounds and pacing slots,
+zero before each): no search reads anything else there, whichever stream it
+comes on and whatever memory the engine was given."""
+import numpy as np
+import pytest
+import torch
+
+import rotormap as rm
+
+pytestmark = pytest.mark.gpu
+
+E4M3_INT = np.array([0xC4, 0xC0, 0xB8, 0x00, 0x38, 0x40, 0x44], np.uint8)  # -3..3
+VALUES = np.arange(-3, 4).astype(np.float32)
+
+
+def integers(seed, rows, rdim=256):
+    """Rows of small integers as e4m3 bytes on the GPU, and their values: every
+    score is a whole number below 2^24, exact in any order of summation."""
+    at = np.random.default_rng(seed).integers(0, 7, size=(rows, rdim))
+    return torch.from_numpy(E4M3_INT[at]).cuda(), VALUES[at]
+
+
+def top(a, b, k):
+    """Top k columns (value descending, equal values by column), 1-based."""
+    sc = a @ b.T
+    loc = np.argsort(-sc, axis=1, kind="stable")[:, :k]
+    return np.take_along_axis(sc, loc, 1), (loc + 1).astype(np.int32)
+
+
+@pytest.mark.parametrize("nb,kernel", [(100, "1sm"), (300, "2sm")])
+def test_new_engine_searches_at_once_on_any_stream(nb, kernel):
+    """Engines made on recycled memory while the default stream is busy, each
+    searched at once on a stream that does not wait for the default one."""
+    A, a = integers(1, nb)
+    B, b = integers(2, 9000)
+    wv, wl = top(a, b, 20)
+    v = torch.empty((nb, 20), device="cuda")
+    l = torch.empty((nb, 20), dtype=torch.int32, device="cuda")
+    side = torch.cuda.Stream()
+    for byte in (0xFF, 0xC0, 0x00, 0x7F, 0x45, 0xC0):
+        # bytes that read as row bounds (large values, NaN) in memory just given back
+        junk = torch.full((256 << 20,), byte, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        del junk
+        torch.cuda.empty_cache()
+        torch.cuda._sleep(40_000_000)
+        eng = rm.TopKEngine(B, k=20, rows_cap=nb, score="f32", kernel=kernel)
+        eng.search(A, nb, None, v, l, side)
+        side.synchronize()
+        assert np.array_equal(v.cpu().numpy(), wv)
+        assert np.array_equal(l.cpu().numpy(), wl)
+        eng.close()
