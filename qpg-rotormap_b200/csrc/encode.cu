@@ -1732,6 +1732,8 @@ extern "C" int r2m_encode_ref_windows(void *dest, int out_kind, float *dest_norm
   R2M_REQUIRE(nwin >= 0, "nwin must be >= 0");
   R2M_REQUIRE(batch_size >= 1, "batch_size must be >= 1");
   if (nwin == 0) return R2M_OK;
+  // one batch holds them all; twice a batch stays within int64
+  batch_size = std::min(batch_size, nwin);
   R2M_REQUIRE(dest && dest_norms && genome && win_pos, "null pointer");
   R2M_REQUIRE(out_kind >= R2M_OUT_F32 && out_kind <= R2M_OUT_E4M3_SCALED, "bad out_kind");
   R2M_REQUIRE(out_kind != R2M_OUT_E4M3_SCALED || dest_scales, "scaled e4m3 needs dest_scales");

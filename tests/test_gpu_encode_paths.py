@@ -123,3 +123,22 @@ def test_bulk_e4m3_at_every_alignment(dtype, src0, dst0, n):
     vals = src[src0:src0 + n].float().cpu().numpy()
     assert np.array_equal(got[dst0:dst0 + n], orc.f32_to_e4m3(vals))
     assert np.all(got[:dst0] == 0x55) and got[-1] == 0x55
+
+
+@pytest.mark.parametrize("batch", [7, 1 << 61, 1 << 62, (1 << 63) - 1])
+@pytest.mark.parametrize("k", [60, 700, 2500])
+def test_any_batch_size_above_the_windows_is_one_batch(batch, k):
+    """Columns of windows in one batch: all forward ones, then all reverse ones."""
+    nwin, s, m, c = 7, 5, 1, 4
+    genome = pack(fragments(np.random.default_rng(k), 6, k + 100).reshape(1, -1))[0]
+    g = torch.from_numpy(np.concatenate([genome, np.zeros(4, np.uint32)]).view(np.int32)).cuda()
+    pos = torch.arange(3, 3 + 17 * nwin, 17, device="cuda")
+    res = []
+    for size in (nwin, batch):
+        out = torch.zeros((2 * nwin, 2 * m * 4 ** c), device="cuda")
+        norms = torch.zeros((2 * nwin, m), device="cuda")
+        check(lib().r2m_encode_ref_windows(ptr(out), 0, ptr(norms), None, ptr(g), ptr(pos), nwin, size, k, s, m, c, 0,
+                                           torch.cuda.current_stream().cuda_stream))
+        res.append((out.cpu().numpy(), norms.cpu().numpy()))
+    assert np.abs(res[0][0]).max() > 0
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
