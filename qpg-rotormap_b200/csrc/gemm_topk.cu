@@ -1369,6 +1369,7 @@ struct Workspace {
   uint32_t *pub;
   float *vals;
   int *cols;
+  size_t zero_bytes;  // slots and bounds, from `pace` on
 };
 static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   unsigned char *p = nullptr;
@@ -1391,6 +1392,7 @@ static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   w->pub = reinterpret_cast<uint32_t *>(p + kPaceSlots * sizeof(long long));
   w->vals = reinterpret_cast<float *>(p + zero);
   w->cols = reinterpret_cast<int *>(p + zero + part);
+  w->zero_bytes = zero;
   return cudaSuccess;
 }
 
@@ -1436,7 +1438,7 @@ struct r2m_engine {
   Workspace ws;
   size_t part_lists;  // capacity in lists (rows x splits)
   size_t pub_lists;   // row bounds the workspace holds
-  bool dirty;         // a launch whose merge did not follow may have left bounds behind
+  bool dirty;         // a launch whose merge did not follow may have left bounds behind, and nothing has cleared them yet
   uint32_t *err;
   int pace_window;    // 0 = no pacing
   bool timing;        // record events around the two kernels of each call
@@ -1651,18 +1653,32 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
   }
   g.pub = (size_t)lists_per_row * g.mpad <= eng->pub_lists ? eng->ws.pub : nullptr;
   g.conc = bound_splits(ctas, g.num_m_tiles, g.splits, halves);
-  // bounds and pacing slots are zero here: the merge of the launch before left
-  // them so, unless it never ran
-  if (eng->dirty)
-    R2M_CUDA(cudaMemsetAsync(eng->ws.pace, 0, kPaceSlots * sizeof(long long) + eng->pub_lists * sizeof(uint32_t), st));
+  // Bounds and pacing slots are zero here: the merge of the launch before left
+  // them so, or the clear that follows a failure did.  Where that failed too,
+  // they are cleared first; a clear that is only being captured runs with the
+  // graph, so the calls after it clear again.
+  auto clear = [&]() { return cudaMemsetAsync(eng->ws.pace, 0, eng->ws.zero_bytes, st); };
+  bool still_dirty = false;
+  if (eng->dirty) {
+    R2M_CUDA(clear());
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    still_dirty = cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  }
   eng->dirty = true;
-  if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[0], st));
-  rc = dispatch_gemm(kind, halves, eng->KT, mapA, plan.bn != BN ? narrow : eng->mapB,
-                     plan.bn != BN ? narrow : eng->mapB128, g, ctas, st);
-  if (rc) return rc;
-  if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[1], st));
-  if ((rc = launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, ctas, st))) return rc;
-  eng->dirty = false;
+  auto launch = [&]() -> int {
+    if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[0], st));
+    if (int e = dispatch_gemm(kind, halves, eng->KT, mapA, plan.bn != BN ? narrow : eng->mapB,
+                              plan.bn != BN ? narrow : eng->mapB128, g, ctas, st))
+      return e;
+    if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[1], st));
+    return launch_merge(g, lists_per_row, eng->KT, d_scaleA, d_vals, d_locs, ctas, st);
+  };
+  rc = launch();
+  if (rc == R2M_OK || clear() == cudaSuccess) eng->dirty = still_dirty;
+  if (rc) {
+    cudaGetLastError();  // of the clear; rc and its message tell what failed first
+    return rc;
+  }
   if (eng->timing) R2M_CUDA(cudaEventRecord(eng->ev[2], st));
   return R2M_OK;
 }

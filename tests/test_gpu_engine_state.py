@@ -50,3 +50,51 @@ def test_new_engine_searches_at_once_on_any_stream(nb, kernel):
         assert np.array_equal(v.cpu().numpy(), wv)
         assert np.array_equal(l.cpu().numpy(), wl)
         eng.close()
+
+
+def captured(eng, A, v, l, ruin=False):
+    """Node types of a search captured on a stream of its own (ruin: the
+    capture is made invalid first, so the search's launch fails)."""
+    from cuda.bindings import driver as drv
+
+    st = torch.cuda.Stream()
+    assert drv.cuStreamBeginCapture(st.cuda_stream, drv.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED)[0] == 0
+    if ruin:
+        assert drv.cuStreamSynchronize(st.cuda_stream)[0] != 0  # refused, and it ends the capture
+    try:
+        eng.search(A, A.shape[0], None, v, l, st)
+    finally:
+        err, g = drv.cuStreamEndCapture(st.cuda_stream)
+    assert err == 0
+    n = drv.cuGraphGetNodes(g, 0)[2]
+    kinds = [drv.cuGraphNodeGetType(x)[1].name.split("_TYPE_")[1] for x in drv.cuGraphGetNodes(g, n)[1][:n]]
+    assert drv.cuGraphDestroy(g)[0] == 0
+    return sorted(kinds)
+
+
+@pytest.mark.parametrize("nb,kernel", [(100, "1sm"), (300, "2sm")])
+def test_a_captured_clear_does_not_stand_for_one_that_ran(nb, kernel):
+    """After a launch that failed, and could not be cleaned up after, every
+    search clears the state until a clear has run: those that are captured as
+    well, one after another, since none of them has run yet."""
+    A, a = integers(3, nb)
+    B, b = integers(4, 5000)
+    wv, wl = top(a, b, 20)
+    eng = rm.TopKEngine(B, k=20, rows_cap=nb, score="f32", kernel=kernel)
+    v = torch.empty((nb, 20), device="cuda")
+    l = torch.empty((nb, 20), dtype=torch.int32, device="cuda")
+
+    def search():
+        eng.search(A, nb, None, v, l)
+        assert np.array_equal(v.cpu().numpy(), wv) and np.array_equal(l.cpu().numpy(), wl)
+
+    search()
+    assert captured(eng, A, v, l) == ["KERNEL", "KERNEL"]
+    with pytest.raises(rm.R2MError):
+        captured(eng, A, v, l, ruin=True)
+    for _ in range(2):
+        assert captured(eng, A, v, l) == ["KERNEL", "KERNEL", "MEMSET"]
+    search()
+    assert captured(eng, A, v, l) == ["KERNEL", "KERNEL"]
+    search()
+    eng.close()
