@@ -85,7 +85,9 @@ int r2m_selftest_bounded_wait(int64_t limit_cycles, int arrive, r2m_stream_t str
  * ([Re; Im] split layout).  dest_norms: (n, m) fp32 (row = fragment), the
  * reference's embeds_norms column per fragment.  dest_scales: n fp32 row
  * scales, required for R2M_OUT_E4M3_SCALED, ignored otherwise (may be NULL).
- * normalize in 0..3.  Requires s <= 16, c <= s, 1 <= m <= 8, k >= s. */
+ * normalize in 0..3.  Requires s <= 16, c <= s, 1 <= m <= 8, k >= s,
+ * m*4^c <= 16384 and 8*m*4^c bytes plus 2.5 bytes a base within 200 KiB (about
+ * 78,600 bases at 1,024 bins). */
 int r2m_encode_frag_real_batch(void *dest, int out_kind, float *dest_norms,
                                float *dest_scales, const uint32_t *dnas,
                                int64_t n, int k, int s, int m, int c,

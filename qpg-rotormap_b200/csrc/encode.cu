@@ -1458,10 +1458,11 @@ static size_t warp_bytes_host(const EncParams &P) {
   return (size_t)P.hist_floats * 4 + (size_t)P.cs_u16 * 2 + (size_t)P.words_u32 * 4 * 2 + 32;
 }
 
+constexpr size_t kSmemCap = 200 * 1024;  // most shared memory of a block of the one-warp paths
+
 template <int OUT, typename KernelFn>
 static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, int *block,
                        size_t *smem, float2 **gtable, cudaStream_t st) {
-  const size_t kSmemCap = 200 * 1024;
   size_t tb = ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
   size_t wb = warp_bytes_host(P);
   P.table_in_smem = (tb + wb * 2 <= 100 * 1024) ? 1 : 0;
@@ -1586,6 +1587,7 @@ static int long_tile(const EncParams &P, int64_t items) {
   const char *force = getenv("R2M_ENCODER");
   if (force && strcmp(force, "dense") == 0) return 0;
   if (P.nw <= 512) return 0;
+  if (warp_bytes_host(P) > kSmemCap) return 0;  // refused, whichever path would be the faster one
   int tile = P.m <= 2 && long_layout(P, 4096).total <= kLongSmem ? 4096 : 0;
   if (tile == 0 && long_layout(P, 2048).total <= kLongSmem) tile = 2048;
   if (tile == 0) return 0;
