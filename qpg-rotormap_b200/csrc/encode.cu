@@ -106,25 +106,32 @@ __device__ __forceinline__ float2 ref_phasor(const EncParams &P, int idm, int p)
   return make_float2(re, im);
 }
 
-// Global table (used when the per-block shared copy does not fit):
-// one thread per (idm, reference chunk) walks the chunk's recurrence.
-__global__ void k_phasor_table(EncParams P, int pitch, float2 *table) {
-  int nchunk = (P.nw + P.Wc - 1) / P.Wc;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nchunk * P.m) return;
-  int idm = t / nchunk, ch = t % nchunk;
-  int p0 = ch * P.Wc, p1 = min(p0 + P.Wc, P.nw);
-  float th = P.theta[idm];
-  float a = th * (float)p0;
+// The same phasors for the windows of reference chunk `ch`, one after another:
+// put(p, phasor of window p).
+template <typename Put>
+__device__ __forceinline__ void phasor_chunk(const EncParams &P, int idm, int ch, Put put) {
+  const int p0 = ch * P.Wc, p1 = min(p0 + P.Wc, P.nw);
+  const float th = P.theta[idm];
+  const float a = th * (float)p0;
   float re = cosf(a), im = sinf(a);
-  float xr = cosf(th), xi = sinf(th);
+  const float xr = cosf(th), xi = sinf(th);
   for (int p = p0; p < p1; ++p) {
-    table[(size_t)idm * pitch + p] = make_float2(re, im);
-    float nr = __fsub_rn(__fmul_rn(re, xr), __fmul_rn(im, xi));
-    float ni = __fadd_rn(__fmul_rn(re, xi), __fmul_rn(im, xr));
+    put(p, make_float2(re, im));
+    const float nr = __fsub_rn(__fmul_rn(re, xr), __fmul_rn(im, xi));
+    const float ni = __fadd_rn(__fmul_rn(re, xi), __fmul_rn(im, xr));
     re = nr;
     im = ni;
   }
+}
+
+// Global table (used when the per-block shared copy does not fit):
+// one thread per (idm, reference chunk) walks the chunk's recurrence.
+__global__ void k_phasor_table(EncParams P, int pitch, float2 *table) {
+  const int nchunk = (P.nw + P.Wc - 1) / P.Wc;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nchunk * P.m) return;
+  const int idm = t / nchunk;
+  phasor_chunk(P, idm, t % nchunk, [&](int p, float2 z) { table[(size_t)idm * pitch + p] = z; });
 }
 
 template <int OUT>
@@ -1200,10 +1207,11 @@ struct LongLayout {
   int order, counts, start, masks, hist, words, misc, total;  // byte offsets (the phasor tile at 0), total bytes
 };
 
-__host__ __device__ inline LongLayout long_layout(const EncParams &P, int TW) {
+// `pitch`: phasors held of each copy, a tile's or (more than one tile) all.
+__host__ __device__ inline LongLayout long_layout(const EncParams &P, int TW, int pitch) {
   const int ncm = 1 << (2 * P.c);
   LongLayout L;
-  L.order = P.m * TW * 8;
+  L.order = P.m * pitch * 8;
   L.counts = L.order + TW * 2;
   L.start = L.counts + kLongWarps * ncm * 2;
   L.masks = L.start + ((ncm * 2 + 2 + 15) & ~15);
@@ -1224,18 +1232,34 @@ __device__ __forceinline__ uint32_t genome_word(const EncParams &P, const uint32
   return v;
 }
 
+// Phasors of windows t0 .. t0 + nt of every copy, by the block.
+__device__ __forceinline__ void form_phasors(const EncParams &P, float2 *tab, int pitch, int t0, int nt) {
+  const int c0 = t0 / P.Wc, nc = (t0 + nt - 1) / P.Wc - c0 + 1;
+  for (int i = threadIdx.x; i < nc * P.m; i += kLongThreads) {
+    const int idm = i / nc;
+    float2 *row = tab + idm * pitch - t0;
+    phasor_chunk(P, idm, c0 + i - idm * nc, [&](int p, float2 z) {
+      if (p >= t0 && p < t0 + nt) row[p] = z;
+    });
+  }
+}
+
 // Item i: fragment i of `src`, or (REF) column i of the index batches over the
 // windows win_pos of the packed genome `src`, the windows' forward columns
-// before their reverse complements within a batch.
-template <int OUT, int TW, bool REF>
-__global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
+// before their reverse complements within a batch.  The phasors come tile by
+// tile from gtable (`pitch` windows a copy), or (FORM) are formed in the block:
+// once where its table of `pitch` windows holds them all, else with every tile.
+template <int OUT, int TW, bool REF, bool FORM>
+__global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
                                                              const int64_t *__restrict__ win_pos, int64_t nwin,
                                                              int64_t batch, int64_t items, void *dest, float *norms,
                                                              float *scales, const float2 *__restrict__ gtable,
                                                              int pitch) {
   constexpr int CW = TW / kLongWarps, NB = CW / 32;  // windows and batches per warp and tile
   extern __shared__ __align__(16) unsigned char smem[];
-  const LongLayout L = long_layout(P, TW);
+  const int held = FORM ? pitch : TW;  // windows of a copy in shared memory
+  const bool whole = FORM && held >= P.nw;
+  const LongLayout L = long_layout(P, TW, held);
   float2 *tab = reinterpret_cast<float2 *>(smem);
   uint16_t *order = reinterpret_cast<uint16_t *>(smem + L.order);
   uint16_t *counts = reinterpret_cast<uint16_t *>(smem + L.counts);
@@ -1251,6 +1275,7 @@ __global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const
   const int ncm = 1 << (2 * P.c), npair = ncm >> 1;
   const size_t rowbytes = (size_t)P.rdim * OutT<OUT>::bytes;
   for (int i = tid; i < kLongWarps * kLongHash; i += kLongThreads) masks[i] = 0u;  // zero between batches
+  if (whole) form_phasors(P, tab, held, 0, P.nw);
   for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
     if constexpr (REF) {
       const int64_t b = it / (2 * batch), off = it - 2 * b * batch;
@@ -1279,12 +1304,16 @@ __global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const
     for (int t0 = 0; t0 < P.nw; t0 += TW) {
       // the tile's phasors, in flight during the sort
       const int nt = min(TW, P.nw - t0), nt2 = (nt + 1) >> 1;
-      for (int idm = 0; idm < P.m; ++idm) {
-        const float2 *g = gtable + (size_t)idm * pitch + t0;
-        for (int i = tid; i < nt2; i += kLongThreads)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tab + idm * TW + 2 * i)),
-                       "l"(g + 2 * i)
-                       : "memory");
+      if constexpr (FORM) {
+        if (!whole) form_phasors(P, tab, held, t0, nt);
+      } else {
+        for (int idm = 0; idm < P.m; ++idm) {
+          const float2 *g = gtable + (size_t)idm * pitch + t0;
+          for (int i = tid; i < nt2; i += kLongThreads)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(tab + idm * TW + 2 * i)),
+                         "l"(g + 2 * i)
+                         : "memory");
+        }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
       uint32_t *c32 = reinterpret_cast<uint32_t *>(counts);
@@ -1385,7 +1414,7 @@ __global__ void __launch_bounds__(kLongThreads) k_encode_long(EncParams P, const
         const int bin = u / P.m, idm = u - bin * P.m;
         const int e0 = start[bin], e1 = start[bin + 1];
         if (e0 == e1) continue;
-        const float2 *tb = tab + idm * TW;
+        const float2 *tb = tab + idm * held + (whole ? t0 : 0);
         float2 *h = reinterpret_cast<float2 *>(hist + hoff(u));
         float2 a = *h;
         int e = e0;
@@ -1460,12 +1489,20 @@ static size_t warp_bytes_host(const EncParams &P) {
 
 constexpr size_t kSmemCap = 200 * 1024;  // most shared memory of a block of the one-warp paths
 
+// Whether a call takes no phasor table in device memory: small ones are formed
+// by every block, so that the call allocates nothing (nor puts allocations into
+// a graph that captures it).
+static bool table_in_block(const EncParams &P) {
+  const size_t tb = ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
+  return tb + warp_bytes_host(P) * 2 <= 100 * 1024;
+}
+
 template <int OUT, typename KernelFn>
 static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, int *block,
                        size_t *smem, float2 **gtable, cudaStream_t st) {
   size_t tb = ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
   size_t wb = warp_bytes_host(P);
-  P.table_in_smem = (tb + wb * 2 <= 100 * 1024) ? 1 : 0;
+  P.table_in_smem = table_in_block(P) ? 1 : 0;
   size_t fixed = P.table_in_smem ? tb : 0;
   int wpb = 8;
   while (wpb > 1 && fixed + wb * wpb > kSmemCap) wpb >>= 1;
@@ -1574,6 +1611,7 @@ static int launch_sparse_ref(const EncParams &P, void *dest, float *norms, float
 }
 
 constexpr int kLongSmem = 220 * 1024;  // most shared memory of a block (the limit set for every launch)
+constexpr int kLongHalf = 113 * 1024;  // most at which two blocks share an SM
 
 // Window tile of the block-per-fragment path for `items` fragments, 0 where
 // the one-warp path is the faster one (or the tile does not fit shared memory:
@@ -1588,8 +1626,8 @@ static int long_tile(const EncParams &P, int64_t items) {
   if (force && strcmp(force, "dense") == 0) return 0;
   if (P.nw <= 512) return 0;
   if (warp_bytes_host(P) > kSmemCap) return 0;  // refused, whichever path would be the faster one
-  int tile = P.m <= 2 && long_layout(P, 4096).total <= kLongSmem ? 4096 : 0;
-  if (tile == 0 && long_layout(P, 2048).total <= kLongSmem) tile = 2048;
+  int tile = P.m <= 2 && long_layout(P, 4096, 4096).total <= kLongSmem ? 4096 : 0;
+  if (tile == 0 && long_layout(P, 2048, 2048).total <= kLongSmem) tile = 2048;
   if (tile == 0) return 0;
   const double sms = sm_count();
   const double block_us = std::ceil(items / (2 * sms)) * (4.0 + 6.0 * ((P.nw + tile - 1) / tile));
@@ -1597,34 +1635,50 @@ static int long_tile(const EncParams &P, int64_t items) {
   return block_us < warp_us ? tile : 0;
 }
 
-template <int OUT, int TW, bool REF>
+template <int OUT, int TW, bool REF, bool FORM>
 static int launch_long_as(const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin, int64_t batch,
                           int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
-  auto kern = k_encode_long<OUT, TW, REF>;
-  const int smem = long_layout(P, TW).total;
+  auto kern = k_encode_long<OUT, TW, REF, FORM>;
+  const int all = (P.nw + 3) & ~1;  // rows start on 16 bytes, and the last pair of a row is whole
+  // a block's own table holds every window as long as two blocks share an SM:
+  // forming each tile's anew takes 1,000 fragments of 5,000 bases at m = 1 81.5
+  // us instead of 75.9, of 2,200 at m = 4 82.0 instead of 57.5 (a table in
+  // device memory: 75.6 and 68.0).  What is left to the tiles: m = 1, c = 5 from
+  // 5,800 bases on (6,500 bases 88.2, a table in device memory 82.1)
+  const int pitch = !FORM || (P.nw > TW && long_layout(P, TW, all).total <= kLongHalf) ? all : TW;
+  const int smem = long_layout(P, TW, FORM ? pitch : TW).total;
   R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem));
   int per_sm = 1;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLongThreads, smem));
   const int64_t cap = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
-  const int pitch = (P.nw + 3) & ~1;  // rows start on 16 bytes, and the last pair of a row is whole
   float2 *gt = nullptr;
-  R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&gt), (size_t)P.m * pitch * sizeof(float2), st));
-  const int tot = (P.nw + P.Wc - 1) / P.Wc * P.m;
-  k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, pitch, gt);
+  if constexpr (!FORM) {
+    R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&gt), (size_t)P.m * pitch * sizeof(float2), st));
+    const int tot = (P.nw + P.Wc - 1) / P.Wc * P.m;
+    k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, pitch, gt);
+  }
   kern<<<(unsigned)(items < cap ? items : cap), kLongThreads, smem, st>>>(P, src, pos, nwin, batch, items, dest, norms,
                                                                          scales, gt, pitch);
   const cudaError_t e = cudaGetLastError();
-  cudaFreeAsync(gt, st);
+  if (gt) cudaFreeAsync(gt, st);
   if (e != cudaSuccess) return cuda_fail(e, "k_encode_long launch");
   return R2M_OK;
+}
+
+template <int OUT, int TW, bool REF>
+static int launch_long_tile(const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin, int64_t batch,
+                            int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
+  return table_in_block(P)
+             ? launch_long_as<OUT, TW, REF, true>(P, src, pos, nwin, batch, items, dest, norms, scales, st)
+             : launch_long_as<OUT, TW, REF, false>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
 }
 
 template <int OUT, bool REF>
 static int launch_long(int tile, const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin,
                        int64_t batch, int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
   if (tile == 4096)
-    return launch_long_as<OUT, 4096, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
-  return launch_long_as<OUT, 2048, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
+    return launch_long_tile<OUT, 4096, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
+  return launch_long_tile<OUT, 2048, REF>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
 }
 
 template <int OUT>

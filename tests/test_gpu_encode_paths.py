@@ -142,3 +142,48 @@ def test_any_batch_size_above_the_windows_is_one_batch(batch, k):
         res.append((out.cpu().numpy(), norms.cpu().numpy()))
     assert np.abs(res[0][0]).max() > 0
     assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
+
+
+def captured(call):
+    """Node types of one encode captured on a stream of its own."""
+    from cuda.bindings import driver as drv
+
+    st = torch.cuda.Stream()
+    call(st.cuda_stream)
+    st.synchronize()
+    assert drv.cuStreamBeginCapture(st.cuda_stream, drv.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED)[0] == 0
+    call(st.cuda_stream)
+    err, g = drv.cuStreamEndCapture(st.cuda_stream)
+    assert err == 0
+    n = drv.cuGraphGetNodes(g, 0)[2]
+    kinds = [drv.cuGraphNodeGetType(x)[1].name.split("_TYPE_")[1] for x in drv.cuGraphGetNodes(g, n)[1][:n]]
+    assert drv.cuGraphDestroy(g)[0] == 0
+    return kinds
+
+
+# windows of one tile and of two, up to the largest phasor table that a block holds
+@pytest.mark.parametrize("k,s,m,c", [(600, 5, 1, 5), (4100, 5, 1, 5), (4101, 5, 1, 5), (6600, 5, 1, 5), (2055, 8, 4, 4),
+                                     (2056, 8, 4, 4), (2200, 8, 4, 4)])
+@pytest.mark.parametrize("ref", [False, True])
+def test_long_fragments_with_a_small_table_allocate_nothing(k, s, m, c, ref, monkeypatch):
+    n = 9
+    codes = fragments(np.random.default_rng(k), n, k)
+    words = torch.from_numpy(pack(codes).view(np.int32)).cuda()
+    genome = torch.from_numpy(np.concatenate([pack(codes.reshape(1, -1))[0], np.zeros(4, np.uint32)]).view(np.int32)).cuda()
+    pos = k * torch.arange(n, dtype=torch.int64, device="cuda")
+    out = torch.empty((2 * n, 2 * m * 4 ** c), device="cuda")
+    norms = torch.empty((2 * n, m), device="cuda")
+
+    def call(stream):
+        if ref:
+            check(lib().r2m_encode_ref_windows(ptr(out), 0, ptr(norms), None, ptr(genome), ptr(pos), n, n, k, s, m, c,
+                                               0, stream))
+        else:
+            check(lib().r2m_encode_frag_real_batch(ptr(out), 0, ptr(norms), None, ptr(words), n, k, s, m, c, 0, stream))
+
+    res = []
+    for path in ("auto", "dense"):
+        monkeypatch.setenv("R2M_ENCODER", path)
+        assert captured(call) == ["KERNEL"]
+        res.append((out[:n].cpu().numpy(), norms[:n].cpu().numpy()))
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
