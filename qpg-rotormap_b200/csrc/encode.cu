@@ -1509,7 +1509,9 @@ static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, in
   if (fixed + wb * wpb > kSmemCap) return fail(R2M_EINVAL, "encoder shared memory does not fit (k or m*4^c too large)");
   *block = 32 * wpb;
   *smem = fixed + wb * wpb;
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+  // the limit is per function, not per launch: the same for every caller, so that
+  // threads encoding with other sizes do not lower it
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
   int per_sm = 0;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, *block, *smem));
   if (per_sm < 1) per_sm = 1;
@@ -1566,9 +1568,7 @@ static int sparse_grid(KernelFn kern, const EncParams &P, int outb, int64_t nwor
   wpb = std::max(1, std::min(wpb, (int)std::max<int64_t>(spread, 8)));
   *block = 32 * wpb;
   *smem = sparse_table_bytes(P) + (size_t)L.warp * wpb;
-  // the limit is per function, not per launch: the same for every caller, so that
-  // threads encoding with other sizes do not lower it
-  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));  // as plan_launch
   int per_sm = 0;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, *block, *smem));
   if (per_sm < 1) per_sm = 1;
@@ -2199,8 +2199,9 @@ extern "C" int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *can
   size_t per = warp_bytes_host(P) + (size_t)P.rdim * 4 + 2 * kMaxCand * 4 + 32;
   P.table_in_smem = (tb + per * 4 <= 200 * 1024) ? 1 : 0;
   size_t smem = (P.table_in_smem ? tb : 0) + per * 4;
-  R2M_REQUIRE(smem <= 220 * 1024, "rescoring shared memory does not fit (k or m*4^c too large)");
-  R2M_CUDA(cudaFuncSetAttribute(k_rescore_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr size_t most = 220 * 1024;
+  R2M_REQUIRE(smem <= most, "rescoring shared memory does not fit (k or m*4^c too large)");
+  R2M_CUDA(cudaFuncSetAttribute(k_rescore_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   float2 *gt = nullptr;
   if (!P.table_in_smem) {
     R2M_CUDA(cudaMallocAsync(&gt, (size_t)P.m * P.nw * sizeof(float2), st));

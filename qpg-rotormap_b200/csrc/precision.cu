@@ -332,8 +332,11 @@ extern "C" int r2m_check_fp64(const uint32_t *d_read_words, int S, const uint32_
   cudaStream_t st = as_stream(stream);
   const long long NC = 32768;
   const size_t smem = smem64_per_warp(P) * kWarps64;
-  R2M_CUDA(cudaFuncSetAttribute(k_encode64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  R2M_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit is per function, not per launch: the most there is for every caller
+  // (more is refused here), so that threads with other sizes do not lower it
+  const int limit = (int)(smem > 227 * 1024 ? smem : 227 * 1024);
+  R2M_CUDA(cudaFuncSetAttribute(k_encode64, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+  R2M_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
   double2 *table = nullptr;
   double *A = nullptr, *Bc = nullptr, *Sc = nullptr;
   void *ws = nullptr;
