@@ -1497,24 +1497,32 @@ static bool table_in_block(const EncParams &P) {
   return tb + warp_bytes_host(P) * 2 <= 100 * 1024;
 }
 
-template <int OUT, typename KernelFn>
-static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, int *block,
-                       size_t *smem, float2 **gtable, cudaStream_t st) {
-  size_t tb = ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15;
-  size_t wb = warp_bytes_host(P);
-  P.table_in_smem = table_in_block(P) ? 1 : 0;
-  size_t fixed = P.table_in_smem ? tb : 0;
-  int wpb = 8;
-  while (wpb > 1 && fixed + wb * wpb > kSmemCap) wpb >>= 1;
-  if (fixed + wb * wpb > kSmemCap) return fail(R2M_EINVAL, "encoder shared memory does not fit (k or m*4^c too large)");
-  *block = 32 * wpb;
-  *smem = fixed + wb * wpb;
+// Warps and shared memory of a block of a one-warp kernel, and the blocks that
+// an SM holds (nothing about P is changed).
+template <typename KernelFn>
+static int one_warp_blocks(const EncParams &P, KernelFn kern, int *wpb, size_t *smem, int *per_sm) {
+  const size_t tb = table_in_block(P) ? ((size_t)P.m * P.nw * 8 + 15) & ~(size_t)15 : 0;
+  const size_t wb = warp_bytes_host(P);
+  *wpb = 8;
+  while (*wpb > 1 && tb + wb * *wpb > kSmemCap) *wpb >>= 1;
+  *smem = tb + wb * *wpb;
+  if (*smem > kSmemCap) return fail(R2M_EINVAL, "encoder shared memory does not fit (k or m*4^c too large)");
   // the limit is per function, not per launch: the same for every caller, so that
   // threads encoding with other sizes do not lower it
   R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
-  int per_sm = 0;
-  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, *block, *smem));
-  if (per_sm < 1) per_sm = 1;
+  *per_sm = 0;
+  R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kern, 32 * *wpb, *smem));
+  if (*per_sm < 1) *per_sm = 1;
+  return R2M_OK;
+}
+
+template <int OUT, typename KernelFn>
+static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, int *block,
+                       size_t *smem, float2 **gtable, cudaStream_t st) {
+  int wpb, per_sm;
+  if (int rc = one_warp_blocks(P, kern, &wpb, smem, &per_sm)) return rc;
+  P.table_in_smem = table_in_block(P) ? 1 : 0;
+  *block = 32 * wpb;
   int64_t want = (nwork + wpb - 1) / wpb;
   int64_t cap = (int64_t)sm_count() * per_sm;
   *grid = (int)(want < cap ? want : cap);
@@ -1613,25 +1621,47 @@ static int launch_sparse_ref(const EncParams &P, void *dest, float *norms, float
 constexpr int kLongSmem = 220 * 1024;  // most shared memory of a block (the limit set for every launch)
 constexpr int kLongHalf = 113 * 1024;  // most at which two blocks share an SM
 
-// Window tile of the block-per-fragment path for `items` fragments, 0 where
-// the one-warp path is the faster one (or the tile does not fit shared memory:
-// over 1,024 c-mers with m > 4).  A block's fragment takes about 4 us and 6 us
-// a tile with two blocks per SM; a warp takes about 1.3 us per 32 windows with
-// 20 resident per SM.  Measured (block against one-warp path, m = 1): 100
-// fragments of 700 bases 24 and 20 us, of 1,000 28 and 43, of 20,000 38 and
-// 506; 8,192 of 1,000 253 and 115, of 2,000 276 and 291, of 5,000 534 and
-// 1,226.  R2M_ENCODER=dense keeps the one-warp path.
-static int long_tile(const EncParams &P, int64_t items) {
+// Window tile of the block-per-fragment path, 0 where the one-warp path (kernel
+// `one_warp`) is the faster one, or the tile does not fit shared memory (the
+// ranks of 16 warps take 32 bytes a c-mer, the histogram 8 a bin): from 4^7 c-mers,
+// (m, c) = (2, 6) and (7, 5) on.  `work` pieces of `each` fragments (an index
+// window is two) go to one warp at a time in the one path, and each fragment to a
+// block in the other.
+//
+// Both run in waves of what the SMs hold at once, and that is where they differ:
+// a block's fragment takes a few us against tens, but an SM holds two blocks, or
+// one (from m = 1 at 4^6 c-mers, m = 2 at 4^5, m = 5 at 4^4, m = 6 below),
+// against up to 32 warps.  What one warp does alone at the end of a fragment (its
+// norms, with normalize 1 to 3 the division of every value as well) weighs the
+// same in both, per wave.  The costs are fitted to measured pairs, 1 to 20,000 fragments of 530
+// to 50,000 bases, m 1 to 8, 4^3 to 4^6 c-mers, normalize 0 to 2, fragments and
+// index windows: the rule takes the slower path by more than 5% in 20 of 2,840, by
+// 17% at most.  Measured, block against one-warp path: 1,000 fragments of 1,000
+// bases at (1, 5) 40 and 25 us, (4, 4) 41 and 33, (2, 5) 60 and 33, with normalize 1
+// 537 and 111; 1,000 of 2,000 at (1, 5) 43 and 44, (2, 5) 64 and 60, (8, 4) 103 and
+// 229; 1,000 of 5,000 at (1, 5) 76 and 192, (4, 4) 116 and 170; 100 of 700 at (1, 5)
+// 12 and 19.
+// R2M_ENCODER=dense keeps the one-warp path.
+template <typename KernelFn>
+static int long_tile(const EncParams &P, KernelFn one_warp, int64_t work, int each) {
   const char *force = getenv("R2M_ENCODER");
   if (force && strcmp(force, "dense") == 0) return 0;
   if (P.nw <= 512) return 0;
-  if (warp_bytes_host(P) > kSmemCap) return 0;  // refused, whichever path would be the faster one
   int tile = P.m <= 2 && long_layout(P, 4096, 4096).total <= kLongSmem ? 4096 : 0;
   if (tile == 0 && long_layout(P, 2048, 2048).total <= kLongSmem) tile = 2048;
   if (tile == 0) return 0;
-  const double sms = sm_count();
-  const double block_us = std::ceil(items / (2 * sms)) * (4.0 + 6.0 * ((P.nw + tile - 1) / tile));
-  const double warp_us = std::ceil(items / (20 * sms)) * 1.3 * ((P.nw + 31) / 32);
+  int wpb, per_sm;
+  size_t smem;
+  if (one_warp_blocks(P, one_warp, &wpb, &smem, &per_sm)) return 0;  // the one-warp path reports what is wrong
+  const double kbins = P.nbin / 1024.0, sms = sm_count();
+  const bool pow2 = (P.m & (P.m - 1)) == 0;
+  const double finish = kbins * (P.normalize ? 36.0 : pow2 ? 2.0 : 11.0);
+  const int blocks = long_layout(P, tile, tile).total <= kLongHalf ? 2 : 1;
+  const double block_us = std::ceil((double)each * work / (blocks * sms)) *
+                          ((P.nw + tile - 1) / tile * (5.0 + 1.2 / 1024 * (1 << (2 * P.c))) + 0.5e-3 * P.nw * P.m + finish);
+  const double batch = (P.m == 4 ? 0.75 : 0.4 + 0.25 * P.m) * (table_in_block(P) ? 1.0 : 1.4);  // of 32 windows
+  const double warp_us = std::ceil(work / (per_sm * wpb * sms)) * each *
+                         ((P.nw + 31) / 32 * batch + 2.0 * kbins + finish);
   return block_us < warp_us ? tile : 0;
 }
 
@@ -1692,7 +1722,7 @@ static int launch_frags(EncParams P, void *dest, float *norms, float *scales, co
       default: return launch_sparse_frags<OUT, 8>(P, dest, norms, scales, dnas, n, st);
     }
   }
-  if (const int tile = long_tile(P, n))
+  if (const int tile = long_tile(P, k_encode_frags<OUT>, n, 1))
     return launch_long<OUT, false>(tile, P, dnas, nullptr, 0, 0, n, dest, norms, scales, st);
   int grid, block;
   size_t smem;
@@ -1717,7 +1747,7 @@ static int launch_ref(EncParams P, void *dest, float *norms, float *scales, cons
       default: return launch_sparse_ref<OUT, 8>(P, dest, norms, scales, genome, pos, nwin, batch, st);
     }
   }
-  if (const int tile = long_tile(P, 2 * nwin))
+  if (const int tile = long_tile(P, k_encode_ref<OUT>, nwin, 2))
     return launch_long<OUT, true>(tile, P, genome, pos, nwin, batch, 2 * nwin, dest, norms, scales, st);
   int grid, block;
   size_t smem;
