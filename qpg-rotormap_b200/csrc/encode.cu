@@ -258,7 +258,7 @@ __device__ __forceinline__ void finish_hist(const EncParams &P, float *hist, flo
   float part[8];
 #pragma unroll
   for (int t = 0; t < 8; ++t) part[t] = 0.f;
-  if (P.m <= 4 && (P.hist_floats & 127) == 0) {
+  if ((P.m <= 2 || P.m == 4) && (P.hist_floats & 127) == 0) {  // (at m = 3 a slot's copies shift from chunk to chunk)
     // walk the histogram linearly in float4 slots (the order of a sum of
     // squares is free): slot s of chunk j holds complex bins 2w', 2w' + 1 of
     // the chunk, w' = s ^ (j % 8), i.e. copies 2(w' & 1) and 2(w' & 1) + 1

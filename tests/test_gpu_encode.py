@@ -305,3 +305,17 @@ def test_sparse_index_windows_equal_dense(monkeypatch):
         assert diff.mean() < 1e-4
         t = orc.e4m3_table()
         assert np.all(np.abs(t[a[diff]] - t[b[diff]]) <= np.abs(t[b[diff]]) * 0.13 + 1e-9)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("c", [1, 2, 3, 4])
+@pytest.mark.parametrize("normalize", [0, 1])
+def test_every_number_of_copies_equals_the_oracle(m, c, normalize):
+    """Rows, norms and per-copy energies of each m, with histograms of part of
+    a chunk and of several."""
+    k, s, n = 150, 8, 6
+    words = random_words(np.random.default_rng(10 * m + c), n, k)
+    emb, norms = _gpu_encode(words, rm.RopeEncoder(k=k, s=s, m=m, c=c), normalize)
+    o32, n32 = orc.rope_f32(words, k, s, m, c, normalize)
+    np.testing.assert_allclose(emb, o32, rtol=RTOL_F32, atol=ATOL_F32)
+    np.testing.assert_allclose(norms, n32, rtol=1e-5, atol=1e-6)
