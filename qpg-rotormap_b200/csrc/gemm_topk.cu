@@ -1370,11 +1370,13 @@ struct Workspace {
   float *vals;
   int *cols;
   size_t zero_bytes;  // slots and bounds, from `pace` on
+  size_t bytes;       // all of it
 };
 static cudaError_t alloc_workspace(size_t lists, int KT, Workspace *w) {
   unsigned char *p = nullptr;
   const size_t part = lists * KT * sizeof(float), zero = kPaceSlots * sizeof(long long) + lists * sizeof(uint32_t);
-  cudaError_t e = cudaMalloc(&p, zero + 2 * part);
+  w->bytes = zero + 2 * part;
+  cudaError_t e = cudaMalloc(&p, w->bytes);
   if (e != cudaSuccess) return e;
   // The first search may come at once and on any stream, and recycled memory
   // read as row bounds drops results: the zeros are in place before this
@@ -1596,7 +1598,7 @@ extern "C" int r2m_engine_info(const r2m_engine *eng, int *k, int *rdim, int *sc
 
 extern "C" int64_t r2m_engine_workspace_bytes(const r2m_engine *eng) {
   if (!eng) return 0;
-  return (int64_t)(eng->part_lists * eng->KT * (sizeof(float) + sizeof(int)));
+  return (int64_t)eng->ws.bytes;
 }
 
 extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const float *d_scaleA, int nb,

@@ -98,3 +98,24 @@ def test_a_captured_clear_does_not_stand_for_one_that_ran(nb, kernel):
     assert captured(eng, A, v, l) == ["KERNEL", "KERNEL"]
     search()
     eng.close()
+
+
+@pytest.mark.parametrize("k,kt", [(5, 8), (20, 20), (64, 64)])
+def test_workspace_bytes_are_all_that_the_engine_allocates(k, kt):
+    """1,024 pacing slots of 8 bytes, and for each partial list a 4-byte row
+    bound and kt values and columns; the allocator hands out whole 2 MiB pages."""
+    B, _ = integers(5, 70_000)
+    torch.cuda.synchronize()
+    a8 = rm.TopKEngine(B, k=k, rows_cap=4000)  # torch's pool holds the staging buffer from here on
+    a8.close()
+    del a8
+    free = torch.cuda.mem_get_info()[0]
+    eng = rm.TopKEngine(B, k=k, rows_cap=4000)
+    held = eng.workspace_bytes
+    assert (held - 8192) % (8 * kt + 4) == 0
+    assert held <= free - torch.cuda.mem_get_info()[0] <= held + (4 << 20)
+    eng.set_tuning(splits=1)  # a schedule that needs less keeps what there is
+    assert eng.workspace_bytes == held
+    eng.set_tuning(splits=64)
+    assert eng.workspace_bytes > held and (eng.workspace_bytes - 8192) % (8 * kt + 4) == 0
+    eng.close()
