@@ -1653,7 +1653,8 @@ extern "C" int r2m_batch_gemm_topk(r2m_engine *eng, const uint8_t *d_A, const fl
     g.pace = eng->ws.pace;
     g.pace_window = eng->pace_window;
   }
-  g.pub = (size_t)lists_per_row * g.mpad <= eng->pub_lists ? eng->ws.pub : nullptr;
+  const size_t bounds = (size_t)lists_per_row * g.mpad;  // indexed with 32 bits
+  g.pub = bounds <= eng->pub_lists && bounds <= INT_MAX ? eng->ws.pub : nullptr;
   g.conc = bound_splits(ctas, g.num_m_tiles, g.splits, halves);
   // Bounds and pacing slots are zero here: the merge of the launch before left
   // them so, or the clear that follows a failure did.  Where that failed too,
