@@ -495,7 +495,9 @@ extern "C" int r2m_server_create(r2m_engine *eng, int k, int s, int m, int c, in
   if (e == cudaSuccess) e = cudaMalloc(&srv->norms, cap * m * 4);
   if (e == cudaSuccess) e = cudaMalloc(&srv->vals, cap * srv->k * 4);
   if (e == cudaSuccess) e = cudaMalloc(&srv->locs, cap * srv->k * 4);
-  if (e == cudaSuccess) e = cudaMemset(srv->a8, 0, cap * srv->rdim);
+  // on the stream that uses it: the default one may be busy when the first
+  // batch comes, and would clear rows already encoded
+  if (e == cudaSuccess) e = cudaMemsetAsync(srv->a8, 0, cap * srv->rdim, srv->comp);
   if (e != cudaSuccess) {
     cudaFree(srv->a8);
     cudaFree(srv->scaleA);

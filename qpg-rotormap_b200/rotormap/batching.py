@@ -199,6 +199,7 @@ class RaggedBatcher:
         self.d_vals = torch.empty((self.cap, k), dtype=torch.float32, device=dev)
         self.d_locs = torch.empty((self.cap, k), dtype=torch.int32, device=dev)
         self.stream = torch.cuda.Stream(dev)
+        self.stream.wait_stream(torch.cuda.current_stream(dev))  # the buffers above and the engine's are filled there
         self.tuner = tuner
         self.use_graphs = use_graphs
         self.graphs: dict = {}

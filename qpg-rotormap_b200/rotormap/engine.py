@@ -360,7 +360,10 @@ class Mapper:
         self.eng, self.re, self.normalize = eng, re, normalize
         dev = eng.device
         cap = eng.rows_cap
-        self.stream = stream or torch.cuda.Stream(dev)
+        self.stream = stream
+        if stream is None:
+            self.stream = torch.cuda.Stream(dev)
+            self.stream.wait_stream(torch.cuda.current_stream(dev))  # the engine's buffers are filled there
         self.h_words = torch.empty((cap, re.words), dtype=torch.int32, pin_memory=True)
         self.h_vals = torch.empty((cap, eng.k), dtype=torch.float32, pin_memory=True)
         self.h_locs = torch.empty((cap, eng.k), dtype=torch.int32, pin_memory=True)

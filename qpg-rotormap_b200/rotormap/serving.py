@@ -216,6 +216,7 @@ def plain_map(eng, re: RopeEncoder, requests, batch: int = 8192, normalize: int 
     until each arrival time (wall-clock replay)."""
     dev = eng.device
     st = torch.cuda.Stream(dev)
+    st.wait_stream(torch.cuda.current_stream(dev))  # the engine's buffers are filled there
     out = []
     W = re.words
     norms = torch.empty((batch, re.m), dtype=torch.float32, device=dev)
