@@ -109,7 +109,12 @@ int r2m_revcomp_frag_words(uint32_t *drc, const uint32_t *dnas, int k,
  * grouped in batches of `batch_size`; batch b (nb windows) fills columns
  * [2*b*batch_size, 2*b*batch_size + nb) with forward windows and the next nb
  * columns with their reverse complements.  dest: (2*nwin, 2*m*4^c) rows of
- * `out_kind`; dest_norms (2*nwin, m); dest_scales 2*nwin (SCALED only). */
+ * `out_kind`; dest_norms (2*nwin, m); dest_scales 2*nwin (SCALED only).  A
+ * batch_size above nwin is one batch.
+ * Both encoders: where 8*m*(k-s+1) + 2*(8*m*4^c + 2.5*k) bytes exceed 100 KiB
+ * (from about 2,300 bases at m = 4, c = 4, 6,600 at m = 1, c = 5) a call
+ * allocates its phasor table stream-ordered, which puts allocation nodes into
+ * a graph that captures it; below, it allocates nothing. */
 int r2m_encode_ref_windows(void *dest, int out_kind, float *dest_norms,
                            float *dest_scales, const uint32_t *genome,
                            const int64_t *win_pos, int64_t nwin,
@@ -239,7 +244,10 @@ int r2m_selftest_noalloc_timeout(int64_t limit_cycles, int nb, int k, float *d_v
  * (genome / col_pos / strand as r2m_encode_ref_windows writes them; strand 1
  * = reverse complement) in fp32 and score the unquantised embeddings' dot
  * product.  scores (nb, kc) in candidate order (may be NULL); out_vals /
- * out_locs (nb, topk) re-ranked, descending, ties by column. */
+ * out_locs (nb, topk) re-ranked, descending, ties by column.  The scores are
+ * the same whichever kernel forms them; normalize 0, k <= 496 and (m, m*4^c) =
+ * (4, 1024), (4, 256), (2, 512), (1, 1024) or (1, 256) take the fast one (six
+ * times the speed). */
 int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *cand, int kc,
                      const uint32_t *genome, const int64_t *col_pos,
                      const uint8_t *strand, int64_t N, int k, int s, int m,

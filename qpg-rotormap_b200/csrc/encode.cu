@@ -1196,9 +1196,9 @@ __global__ void __launch_bounds__(32 * sparse_warps(M, OutT<OUT>::bytes),
 // order, from the tile's phasors in shared memory.  Bins keep their
 // running sums in the dense histogram, whose norms and output pass are
 // those of the one-warp path.  Counts are 16-bit pairs: TW < 65536.
-// What bounds it is issue (63% of cycles, 120,000 warp instructions per 20,000
-// bases).  1,000 fragments of 20,000 bases, s5 m1 c5: 1,657 -> 213 us; s8 m4 c4:
-// 1,765 -> 394 us.
+// What bounds it is issue (64% of cycles, 123,000 warp instructions per 20,000
+// bases).  1,000 fragments of 20,000 bases, s5 m1 c5: 1,657 -> 206 us; s8 m4 c4:
+// 1,765 -> 388 us.
 constexpr int kLongWarps = 16;
 constexpr int kLongThreads = 32 * kLongWarps;
 constexpr int kLongHash = 256;  // lane masks per warp (c-mers that share one are told apart by shuffles)
@@ -1249,6 +1249,9 @@ __device__ __forceinline__ void form_phasors(const EncParams &P, float2 *tab, in
 // before their reverse complements within a batch.  The phasors come tile by
 // tile from gtable (`pitch` windows a copy), or (FORM) are formed in the block:
 // once where its table of `pitch` windows holds them all, else with every tile.
+// Two blocks per SM need 64 registers a thread, which fp16 rows and FORM exceed
+// unless all are held to them (1,000 x 20,000 bases: fp16 rows 219 -> 199 us, e4m3
+// 197.8 -> 198.6; left to take what they like, one block per SM, 220).
 template <int OUT, int TW, bool REF, bool FORM>
 __global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
                                                              const int64_t *__restrict__ win_pos, int64_t nwin,
@@ -1447,11 +1450,11 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, co
 
 // Bulk conversion, 16 values per thread and step.  VEC (both pointers 16-byte
 // aligned): 16-byte loads, all in flight before the first conversion, and one
-// 16-byte store, so a step moves 48 (fp16) or 80 (fp32) bytes per thread and
-// the pass is bound by HBM: 8,192 x 2,048 fp16 values in 10.9 us (4.6 TB/s,
-// launch included), against 63.5 us with one value per load and one byte per
-// store.  Other alignments and the tail take one value at a time, consecutive
-// lanes on consecutive values.
+// 16-byte store, so a step moves 48 (fp16) or 80 (fp32) bytes per thread.
+// 65,536 x 2,048 fp16 values are bound by HBM, 61.2 us (6.6 TB/s); 8,192 x 2,048
+// fit in L2 and take 10.4, the cost of a call, against 63.5 with one value per
+// load and one byte per store.  Other alignments and the tail take one value at
+// a time, consecutive lanes on consecutive values.
 __device__ __forceinline__ float widen(float x) { return x; }
 __device__ __forceinline__ float widen(__half x) { return __half2float(x); }
 
@@ -1983,9 +1986,11 @@ __global__ void __launch_bounds__(128) k_rescore_fp32(EncParams P, const uint32_
   }
 }
 
-// The same for the encoders in use (normalize = 0, m = 1, 2 or 4, 256, 512 or
-// 1024 bins, fragments of at most 496 bases): one block of four warps per
-// read, the candidates dealt out to its warps.  What bounds it is instruction
+// The same for the encoders in use (normalize = 0, fragments of at most 496
+// bases, (m, bins) = (4, 1024), (4, 256), (2, 512), (1, 1024) or (1, 256): the bins
+// of a lane are unrolled, so every number of them is a kernel of its own): one
+// block of four warps per read, the candidates dealt out to its warps.  Other
+// encoders take the general kernel above, with the same scores.  What bounds it is instruction
 // issue: a candidate is a whole encode (nw windows) and a dot product over
 // every bin, against a few hundred bytes of memory traffic.  So
 //   * the read's embedding is formed once per block, in shared memory: kept

@@ -1130,7 +1130,11 @@ static size_t gemm_smem_bytes(int H) {
 // 6.5 us up to 20 entries, 50 at 64), so the splits minimise waves x (tiles +
 // fixed); 6% per doubling of the waves covers the index reads that pairs in
 // different splits do not share (8,192 x 619,001: 7.2 ms with 2 splits in one
-// wave, 7.6 with 9 in four).  Against the rule before (at least four units per CTA, capped at 64
+// wave, 7.6 with 9 in four).  Its weight falls as units grow, and 8,192 reads take
+// 9 splits again from 3.3 million columns on, where they are the faster: 4,194,304
+// 49.0 ms (2 splits 50.7), 16,777,216 193.9 (202.8); 4,096 reads with 9 98.2 (4
+// splits 102.7), 5,120 with 11 120.6 (3 splits 132.1), 7,168 with 5 171.9 (2 splits
+// 189.5).  Against the rule before (at least four units per CTA, capped at 64
 // splits): 100 reads x 1,000,003 columns 489 -> 336 us (148 splits, one per
 // SM), 1,000 x 300,007 575 -> 498 (18), 1,000 x 30,000 196 -> 103 (18),
 // 4,096 x 20,000 333 -> 182 (4), 4,096 x 500,000 at k = 64 4.9 -> 3.6 ms (4).

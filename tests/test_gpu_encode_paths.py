@@ -1,5 +1,5 @@
 """The encoder's dispatch: the block-per-fragment path for long fragments, the
-register path of the FP32 rescoring and the bulk e4m3 conversion give the bytes
+block-per-read path of the FP32 rescoring and the bulk e4m3 conversion give the bytes
 of the general path they stand in for, at the edges of their tiles and on
 fragments whose windows crowd into few bins."""
 import numpy as np
