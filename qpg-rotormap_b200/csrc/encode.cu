@@ -1533,7 +1533,7 @@ static int plan_launch(EncParams &P, KernelFn kern, int64_t nwork, int *grid, in
   *gtable = nullptr;
   if (!P.table_in_smem) {
     float2 *t = nullptr;
-    R2M_CUDA(cudaMallocAsync(&t, (size_t)P.m * P.nw * sizeof(float2), st));
+    R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&t), (size_t)P.m * P.nw * sizeof(float2), st));
     int nchunk = (P.nw + P.Wc - 1) / P.Wc;
     int tot = nchunk * P.m;
     k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, P.nw, t);
@@ -2239,7 +2239,7 @@ extern "C" int r2m_rescore_fp32(const uint32_t *dnas, int nb, const int32_t *can
   R2M_CUDA(cudaFuncSetAttribute(k_rescore_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   float2 *gt = nullptr;
   if (!P.table_in_smem) {
-    R2M_CUDA(cudaMallocAsync(&gt, (size_t)P.m * P.nw * sizeof(float2), st));
+    R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&gt), (size_t)P.m * P.nw * sizeof(float2), st));
     int nchunk = (P.nw + P.Wc - 1) / P.Wc;
     k_phasor_table<<<(nchunk * P.m + 127) / 128, 128, 0, st>>>(P, P.nw, gt);
   }
