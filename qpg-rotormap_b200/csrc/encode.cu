@@ -1246,22 +1246,25 @@ __device__ __forceinline__ void form_phasors(const EncParams &P, float2 *tab, in
 
 // Item i: fragment i of `src`, or (REF) column i of the index batches over the
 // windows win_pos of the packed genome `src`, the windows' forward columns
-// before their reverse complements within a batch.  The phasors come tile by
-// tile from gtable (`pitch` windows a copy), or (FORM) are formed in the block:
-// once where its table of `pitch` windows holds them all, else with every tile.
-// Two blocks per SM need 64 registers a thread, which fp16 rows and FORM exceed
-// unless all are held to them (1,000 x 20,000 bases: fp16 rows 219 -> 199 us, e4m3
-// 197.8 -> 198.6; left to take what they like, one block per SM, 220).
-template <int OUT, int TW, bool REF, bool FORM>
-__global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
+// before their reverse complements within a batch.  `pitch`: phasors of a copy
+// in gtable (FROM_MEMORY) or held by the block.
+// Two blocks per SM need 64 registers a thread.  fp16 rows and the forms that
+// compute phasors are held to them (1,000 x 20,000 bases to fp16 219 -> 199 us);
+// the others stay there by themselves (0: no bound given), 0.5% faster than held.
+enum PhasorSource {
+  FROM_MEMORY,    // tile by tile from a table in device memory
+  HELD,           // formed once by the block, which holds those of every window
+  FORMED_BY_TILE  // formed by the block with every tile
+};
+template <int OUT, int TW, bool REF, PhasorSource SRC>
+__global__ void __launch_bounds__(kLongThreads, SRC != FROM_MEMORY || OUT == R2M_OUT_F16 ? 2 : 0) k_encode_long(EncParams P, const uint32_t *__restrict__ src,
                                                              const int64_t *__restrict__ win_pos, int64_t nwin,
                                                              int64_t batch, int64_t items, void *dest, float *norms,
                                                              float *scales, const float2 *__restrict__ gtable,
                                                              int pitch) {
   constexpr int CW = TW / kLongWarps, NB = CW / 32;  // windows and batches per warp and tile
   extern __shared__ __align__(16) unsigned char smem[];
-  const int held = FORM ? pitch : TW;  // windows of a copy in shared memory
-  const bool whole = FORM && held >= P.nw;
+  const int held = SRC == HELD ? pitch : TW;  // windows of a copy in shared memory
   const LongLayout L = long_layout(P, TW, held);
   float2 *tab = reinterpret_cast<float2 *>(smem);
   uint16_t *order = reinterpret_cast<uint16_t *>(smem + L.order);
@@ -1278,7 +1281,7 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, co
   const int ncm = 1 << (2 * P.c), npair = ncm >> 1;
   const size_t rowbytes = (size_t)P.rdim * OutT<OUT>::bytes;
   for (int i = tid; i < kLongWarps * kLongHash; i += kLongThreads) masks[i] = 0u;  // zero between batches
-  if (whole) form_phasors(P, tab, held, 0, P.nw);
+  if constexpr (SRC == HELD) form_phasors(P, tab, held, 0, P.nw);
   for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
     if constexpr (REF) {
       const int64_t b = it / (2 * batch), off = it - 2 * b * batch;
@@ -1307,9 +1310,9 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, co
     for (int t0 = 0; t0 < P.nw; t0 += TW) {
       // the tile's phasors, in flight during the sort
       const int nt = min(TW, P.nw - t0), nt2 = (nt + 1) >> 1;
-      if constexpr (FORM) {
-        if (!whole) form_phasors(P, tab, held, t0, nt);
-      } else {
+      if constexpr (SRC == FORMED_BY_TILE) {
+        form_phasors(P, tab, held, t0, nt);
+      } else if constexpr (SRC == FROM_MEMORY) {
         for (int idm = 0; idm < P.m; ++idm) {
           const float2 *g = gtable + (size_t)idm * pitch + t0;
           for (int i = tid; i < nt2; i += kLongThreads)
@@ -1417,7 +1420,7 @@ __global__ void __launch_bounds__(kLongThreads, 2) k_encode_long(EncParams P, co
         const int bin = u / P.m, idm = u - bin * P.m;
         const int e0 = start[bin], e1 = start[bin + 1];
         if (e0 == e1) continue;
-        const float2 *tb = tab + idm * held + (whole ? t0 : 0);
+        const float2 *tb = tab + idm * held + (SRC == HELD ? t0 : 0);
         float2 *h = reinterpret_cast<float2 *>(hist + hoff(u));
         float2 a = *h;
         int e = e0;
@@ -1624,6 +1627,21 @@ static int launch_sparse_ref(const EncParams &P, void *dest, float *norms, float
 constexpr int kLongSmem = 220 * 1024;  // most shared memory of a block (the limit set for every launch)
 constexpr int kLongHalf = 113 * 1024;  // most at which two blocks share an SM
 
+// Where the phasors come from, and how many of a copy a block holds.  Tables that
+// fit a block are formed there: every window's, unless that leaves an SM one block
+// where a tile's would leave it two, which is m = 1, c = 5 from 5,819 bases on
+// (1,000 fragments of 6,500 bases 88 us by tile, with a table in device memory 82).
+static PhasorSource phasor_source(const EncParams &P, int TW, int *held) {
+  *held = TW;
+  if (!table_in_block(P)) return FROM_MEMORY;
+  if (P.nw <= TW) return HELD;
+  const int all = (P.nw + 3) & ~1;
+  if (TW == 4096 && long_layout(P, TW, all).total > kLongHalf && long_layout(P, TW, TW).total <= kLongHalf)
+    return FORMED_BY_TILE;
+  *held = all;
+  return HELD;
+}
+
 // Window tile of the block-per-fragment path, 0 where the one-warp path (kernel
 // `one_warp`) is the faster one, or the tile does not fit shared memory (the
 // ranks of 16 warps take 32 bytes a c-mer, the histogram 8 a bin): from 4^7 c-mers,
@@ -1659,7 +1677,9 @@ static int long_tile(const EncParams &P, KernelFn one_warp, int64_t work, int ea
   const double kbins = P.nbin / 1024.0, sms = sm_count();
   const bool pow2 = (P.m & (P.m - 1)) == 0;
   const double finish = kbins * (P.normalize ? 36.0 : pow2 ? 2.0 : 11.0);
-  const int blocks = long_layout(P, tile, tile).total <= kLongHalf ? 2 : 1;
+  int held;
+  phasor_source(P, tile, &held);
+  const int blocks = long_layout(P, tile, held).total <= kLongHalf ? 2 : 1;
   const double block_us = std::ceil((double)each * work / (blocks * sms)) *
                           ((P.nw + tile - 1) / tile * (5.0 + 1.2 / 1024 * (1 << (2 * P.c))) + 0.5e-3 * P.nw * P.m + finish);
   const double batch = (P.m == 4 ? 0.75 : 0.4 + 0.25 * P.m) * (table_in_block(P) ? 1.0 : 1.4);  // of 32 windows
@@ -1668,24 +1688,19 @@ static int long_tile(const EncParams &P, KernelFn one_warp, int64_t work, int ea
   return block_us < warp_us ? tile : 0;
 }
 
-template <int OUT, int TW, bool REF, bool FORM>
-static int launch_long_as(const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin, int64_t batch,
-                          int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
-  auto kern = k_encode_long<OUT, TW, REF, FORM>;
-  const int all = (P.nw + 3) & ~1;  // rows start on 16 bytes, and the last pair of a row is whole
-  // a block's own table holds every window as long as two blocks share an SM:
-  // forming each tile's anew takes 1,000 fragments of 5,000 bases at m = 1 81.5
-  // us instead of 75.9, of 2,200 at m = 4 82.0 instead of 57.5 (a table in
-  // device memory: 75.6 and 68.0).  What is left to the tiles: m = 1, c = 5 from
-  // 5,800 bases on (6,500 bases 88.2, a table in device memory 82.1)
-  const int pitch = !FORM || (P.nw > TW && long_layout(P, TW, all).total <= kLongHalf) ? all : TW;
-  const int smem = long_layout(P, TW, FORM ? pitch : TW).total;
+template <int OUT, int TW, bool REF, PhasorSource SRC>
+static int launch_long_as(const EncParams &P, int held, const uint32_t *src, const int64_t *pos, int64_t nwin,
+                          int64_t batch, int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
+  auto kern = k_encode_long<OUT, TW, REF, SRC>;
+  const int smem = long_layout(P, TW, held).total;
   R2M_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kLongSmem));
   int per_sm = 1;
   R2M_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLongThreads, smem));
   const int64_t cap = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
+  int pitch = held;
   float2 *gt = nullptr;
-  if constexpr (!FORM) {
+  if constexpr (SRC == FROM_MEMORY) {
+    pitch = (P.nw + 3) & ~1;  // rows start on 16 bytes, and the last pair of a row is whole
     R2M_CUDA(pool_alloc(reinterpret_cast<void **>(&gt), (size_t)P.m * pitch * sizeof(float2), st));
     const int tot = (P.nw + P.Wc - 1) / P.Wc * P.m;
     k_phasor_table<<<(tot + 127) / 128, 128, 0, st>>>(P, pitch, gt);
@@ -1701,9 +1716,15 @@ static int launch_long_as(const EncParams &P, const uint32_t *src, const int64_t
 template <int OUT, int TW, bool REF>
 static int launch_long_tile(const EncParams &P, const uint32_t *src, const int64_t *pos, int64_t nwin, int64_t batch,
                             int64_t items, void *dest, float *norms, float *scales, cudaStream_t st) {
-  return table_in_block(P)
-             ? launch_long_as<OUT, TW, REF, true>(P, src, pos, nwin, batch, items, dest, norms, scales, st)
-             : launch_long_as<OUT, TW, REF, false>(P, src, pos, nwin, batch, items, dest, norms, scales, st);
+  int held;
+  const PhasorSource from = phasor_source(P, TW, &held);
+  if constexpr (TW == 4096) {
+    if (from == FORMED_BY_TILE)
+      return launch_long_as<OUT, TW, REF, FORMED_BY_TILE>(P, held, src, pos, nwin, batch, items, dest, norms, scales, st);
+  }
+  return from == HELD
+             ? launch_long_as<OUT, TW, REF, HELD>(P, held, src, pos, nwin, batch, items, dest, norms, scales, st)
+             : launch_long_as<OUT, TW, REF, FROM_MEMORY>(P, held, src, pos, nwin, batch, items, dest, norms, scales, st);
 }
 
 template <int OUT, bool REF>
